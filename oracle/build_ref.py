@@ -43,10 +43,10 @@ MOUNTED_SRC = "/root/reference"
 
 
 def locate():
-    """The reference source tree to build from, or None when it is absent
-    (the GPU hosts carry only the built modules)."""
+    """The reference source tree to build from, or None when it is absent or
+    empty (the GPU hosts carry only the built modules)."""
     src = os.environ.get("OEC_REFERENCE", MOUNTED_SRC)
-    return src if os.path.isdir(src) else None
+    return src if os.path.isfile(os.path.join(src, "poissonSolver.pyx")) else None
 
 MODULES = ["constants", "randomGen", "specFun", "grid", "particles", "particleBoundary",
            "kdTree", "particleManagement", "particleEmitter", "poissonSolver", "magneticField", "util",
