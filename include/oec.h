@@ -424,6 +424,52 @@ int oec_cell_merge(const oec_grid_t *grid, oec_particles_t *p, int32_t n_cand, i
 
 /* ------------------------------------------------ Poisson solve (A15-A16) */
 
+/* Nested-dissection fronts of A (nd_setup.py): the form in which the direct
+ * solve normally runs.  A front has s pivots and b boundary unknowns (pivots of
+ * fronts above it); its blocks are X = A11^-1 and G = A21 X, stored input by
+ * input: [X | G^T] as s rows of ldf values from mat + mf, G as b rows of ldb
+ * values from mat + mb (ldf, ldb, mf, mb even).  Level 0 is the one front at the
+ * root; forward runs from level n_levels - 1 to 0, backward from 1 on.  A tile
+ * is (front, first output); width 8, 16, 32 or 64 outputs are a CTA's work, width
+ * 0 gives a whole front (at most 256 inputs) to a warp.  piv_src / bnd_src hold,
+ * per pivot / boundary entry, up to four entries of u that its children left
+ * for it (-1: none).  Pointers are device pointers (host ones in
+ * oec_lu_host_t). */
+#define OEC_ND_MAX_LEVELS 16
+#define OEC_ND_MAX_FRONT 6144
+typedef struct oec_nd_front {
+    int32_t s, b;
+    int32_t piv0, bnd0;        /* first entry in piv_node / bnd_node (and y / u) */
+    int32_t ldf, ldb;
+    int64_t mf, mb;
+} oec_nd_front_t;
+typedef struct oec_nd_level {
+    int32_t fwd_tile, fwd_tiles, fwd_width;
+    int32_t bwd_tile, bwd_tiles, bwd_width;
+    int32_t has_children;      /* some front of the level has fronts below it */
+    int32_t pad;
+} oec_nd_level_t;
+typedef struct oec_nd {
+    int32_t n;                 /* unknowns */
+    int32_t n_nodes;           /* grid nodes (phi length) */
+    int32_t n_bnd;             /* boundary entries of all fronts */
+    int32_t n_outside;         /* nodes that are no unknown (phi = 0) */
+    int32_t n_levels;
+    int32_t max_front;         /* largest s or b */
+    int32_t n_fronts;
+    int32_t n_tiles;
+    int64_t n_mat;
+    oec_nd_level_t level[OEC_ND_MAX_LEVELS];
+    const oec_nd_front_t *fronts; /* [n_fronts] */
+    const int32_t *tiles;      /* [2 * n_tiles] */
+    const int32_t *piv_node;   /* [n] */
+    const int32_t *piv_src;    /* [4 * n] */
+    const int32_t *bnd_node;   /* [n_bnd] */
+    const int32_t *bnd_src;    /* [4 * n_bnd] */
+    const int32_t *outside;    /* [n_outside] */
+    const double *mat;         /* [n_mat] */
+} oec_nd_t;
+
 /* Device form of SuperLU's P_r A P_c = L U (poissonSolver.pyx:59).
  * Rows [0, head) of each factor are solved level by level; the last
  * m = n - head rows ("tail") use dense inverses of their triangular blocks.
@@ -452,6 +498,8 @@ typedef struct oec_lu {
     const int32_t *u_rows;     /* [head] */
     const int32_t *u_ptr, *u_idx; const double *u_val;    /* strict upper U, head rows in level order */
     const double *u_diag;      /* [head] diagonal of U, in level order */
+    const oec_nd_t *nd;        /* HOST struct or NULL: when given the solve runs on these fronts, and of the other
+                                  fields only n, n_nodes and head_path (which must be valid) are read */
     const double *tu_inv;      /* [m*m] inverse of U[tail,tail], row-major */
     int32_t head_path;         /* how the head levels run: OEC_LU_HEAD_* (0: chosen by size) */
     const int8_t *l_level_lanes; /* HOST [l_nlevels] or NULL: per level, 0 or the lanes per row (1, 2, 4, ..., 32)
@@ -475,7 +523,8 @@ typedef struct oec_lu {
 #define OEC_LU_HEAD_ONE_CTA 3      /* one CTA per factor, the vector in shared memory */
 
 /* phi = A^-1 q on the inside nodes, 0 elsewhere (poissonSolver.pyx:85).
- * q_dev, phi_dev: [n_nodes]; work_dev: n + (n - head) doubles. */
+ * q_dev, phi_dev: [n_nodes]; work_dev: n + (n - head) doubles, or with nd
+ * n + nd->n_bnd. */
 int oec_lu_solve(const oec_lu_t *lu, const double *q_dev, double *phi_dev, double *work_dev, void *stream);
 
 /* y = A x, CSR with int32 indices (E = phiToE . phi, poissonSolver.pyx:87). */
@@ -485,6 +534,13 @@ int oec_spmv_csr(int32_t nrows, const int32_t *ptr_dev, const int32_t *idx_dev, 
 /* Host helper: dependency level of each row of a triangular CSR factor. */
 int oec_trsv_levels(int32_t nrows, const int32_t *ptr, const int32_t *idx, int32_t lower, int32_t ncols_dep,
                     int32_t *level_out, int32_t *nlevels_out);
+
+/* Host helper: nested dissection of n unknowns at the grid positions (ix, iy)
+ * by grid lines, to depth max_depth or sets of at most `leaf` unknowns:
+ * node_out[i] is the number of unknown i's node of the binary tree (root 1,
+ * children 2h and 2h + 1). */
+int oec_nd_dissect(int64_t n, const int32_t *ix, const int32_t *iy, int32_t max_depth, int32_t leaf,
+                   int64_t *node_out);
 
 /* ---------------------------------------- iterative Poisson solve (A16) */
 
@@ -784,7 +840,8 @@ int oec_status(oec_ctx_t *ctx, oec_status_t *out);
  * the host-side setup (SuperLU's factors, poissonSolver.pyx:59, in the
  * head/tail form; tl_inv/tu_inv the dense inverses of the tail blocks).
  * Sizes: rhs_node/sol_src/sol_node n; l_rows/u_rows/u_diag head; l_ptr/u_ptr
- * head+1 (nnz = ptr[head]); lc_ptr m+1 (m = n - head); tl_inv/tu_inv m*m. */
+ * head+1 (nnz = ptr[head]); lc_ptr m+1 (m = n - head); tl_inv/tu_inv m*m.
+ * With nd, nd's arrays alone are read. */
 typedef oec_lu_t oec_lu_host_t;
 
 /* One buildup run (example01_basic.py:36-97).  HOST arrays, copied by

@@ -14,7 +14,7 @@ from . import _lib, constants  # noqa: F401
 
 __all__ = ["constants", "grid", "particles", "particleBoundary", "particleEmitter", "poissonSolver", "grid_geom",
            "magneticField", "util", "beam", "buildup", "batch", "autotune", "checkpoint", "shard", "session",
-           "lu_setup", "furman", "cnn", "particleManagement"]
+           "lu_setup", "nd_setup", "furman", "cnn", "particleManagement"]
 
 
 def __getattr__(name):

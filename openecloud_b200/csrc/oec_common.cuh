@@ -94,6 +94,9 @@ int per_device_cached(std::atomic<int> *slots, F compute) {
 // Number of SMs of the current device (cached per device).
 int sm_count();
 
+// The direct solve on nested-dissection fronts (nd_solve.cu).
+int nd_solve(const oec_nd_t *nd, const double *q, double *phi, double *work, cudaStream_t s);
+
 // Programmatic dependent launch.  A kernel launched by launch_overlapped may
 // be scheduled while the kernel before it on the stream (or before it in a
 // captured graph) still runs; its first statement is pdl_wait(), which

@@ -471,6 +471,12 @@ extern "C" int oec_lu_solve(const oec_lu_t *lu, const double *q_dev, double *phi
                             void *stream) {
     if (!lu || !q_dev || !phi_dev || !work_dev || lu->n <= 0 || lu->head < 0 || lu->head > lu->n)
         return OEC_ERR_INVALID;
+    if (lu->nd) {
+        if (lu->head_path < OEC_LU_HEAD_AUTO || lu->head_path > OEC_LU_HEAD_ONE_CTA || lu->nd->n != lu->n ||
+            lu->nd->n_nodes != lu->n_nodes)
+            return OEC_ERR_INVALID;
+        return nd_solve(lu->nd, q_dev, phi_dev, work_dev, as_stream(stream));
+    }
     const int n = lu->n, h = lu->head, m = n - h;
     if (m > 0 && (!lu->tl_inv || !lu->tu_inv)) return OEC_ERR_INVALID;
     cudaStream_t s = as_stream(stream);

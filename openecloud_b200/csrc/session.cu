@@ -92,6 +92,7 @@ struct oec_run {
     double *wscale = nullptr, *rho = nullptr, *phi = nullptr, *efield = nullptr, *lu_work = nullptr;
     float *etab = nullptr;
     oec_lu_t lu{};
+    oec_nd_t nd{};
     std::vector<int32_t> l_level_ptr, u_level_ptr;
     std::vector<int8_t> l_lanes, u_lanes;
     int32_t *e_ptr = nullptr, *e_idx = nullptr;
@@ -217,8 +218,10 @@ bool valid_desc(const oec_run_desc_t *d) {
            d->beam_table && d->beam_profile && d->target >= 1 && d->management_every >= 1 &&
            (d->boundary_kind == OEC_BOUNDARY_RECT || d->boundary_kind == OEC_BOUNDARY_ELLIPSE) &&
            (d->type_b == 0 || d->type_b == 1) && d->mass > 0 && L.n >= 1 && L.head >= 0 && L.head <= L.n &&
-           L.n_nodes == d->grid.nx * d->grid.ny && L.l_level_ptr && L.u_level_ptr && d->e_ptr && d->e_idx &&
-           d->e_val && L.rhs_node && L.sol_src && L.sol_node;
+           L.n_nodes == d->grid.nx * d->grid.ny && d->e_ptr && d->e_idx && d->e_val &&
+           (L.nd ? L.nd->n == L.n && L.nd->n_nodes == L.n_nodes && L.nd->n_fronts >= 1 && L.nd->n_tiles >= 1 &&
+                       L.nd->n_bnd >= 0 && L.nd->n_outside >= 0 && L.nd->n_mat >= 1
+                 : L.l_level_ptr && L.u_level_ptr && L.rhs_node && L.sol_src && L.sol_node);
 }
 
 int create_run(oec_ctx *c, const oec_run_desc_t *d, oec_run *r) {
@@ -258,43 +261,59 @@ int create_run(oec_ctx *c, const oec_run_desc_t *d, oec_run *r) {
     r->lu.head_path = L.head_path;
     int32_t *i32;
     double *f64;
-    OEC_TRY(ctx_upload(c, L.rhs_node, L.n, &i32)); r->lu.rhs_node = i32;
-    OEC_TRY(ctx_upload(c, L.sol_src, L.n, &i32)); r->lu.sol_src = i32;
-    OEC_TRY(ctx_upload(c, L.sol_node, L.n, &i32)); r->lu.sol_node = i32;
-    r->lu.l_nlevels = L.l_nlevels;
-    r->lu.u_nlevels = L.u_nlevels;
-    r->l_level_ptr.assign(L.l_level_ptr, L.l_level_ptr + L.l_nlevels + 1);
-    r->u_level_ptr.assign(L.u_level_ptr, L.u_level_ptr + L.u_nlevels + 1);
-    r->lu.l_level_ptr = r->l_level_ptr.data();
-    r->lu.u_level_ptr = r->u_level_ptr.data();
-    if (L.l_level_lanes) {
-        r->l_lanes.assign(L.l_level_lanes, L.l_level_lanes + L.l_nlevels);
-        r->lu.l_level_lanes = r->l_lanes.data();
+    if (L.nd) {
+        r->nd = *L.nd;
+        const oec_nd_t &h = *L.nd;
+        oec_nd_front_t *fr;
+        OEC_TRY(ctx_upload(c, h.fronts, h.n_fronts, &fr)); r->nd.fronts = fr;
+        OEC_TRY(ctx_upload(c, h.tiles, 2 * (size_t)h.n_tiles, &i32)); r->nd.tiles = i32;
+        OEC_TRY(ctx_upload(c, h.piv_node, h.n, &i32)); r->nd.piv_node = i32;
+        OEC_TRY(ctx_upload(c, h.piv_src, 4 * (size_t)h.n, &i32)); r->nd.piv_src = i32;
+        OEC_TRY(ctx_upload(c, h.bnd_node, h.n_bnd, &i32)); r->nd.bnd_node = i32;
+        OEC_TRY(ctx_upload(c, h.bnd_src, 4 * (size_t)h.n_bnd, &i32)); r->nd.bnd_src = i32;
+        OEC_TRY(ctx_upload(c, h.outside, h.n_outside, &i32)); r->nd.outside = i32;
+        OEC_TRY(ctx_upload(c, h.mat, h.n_mat, &f64)); r->nd.mat = f64;
+        r->lu.nd = &r->nd;
+        OEC_TRY(ctx_array(c, (size_t)h.n + h.n_bnd + 1, &r->lu_work));
+    } else {
+        OEC_TRY(ctx_upload(c, L.rhs_node, L.n, &i32)); r->lu.rhs_node = i32;
+        OEC_TRY(ctx_upload(c, L.sol_src, L.n, &i32)); r->lu.sol_src = i32;
+        OEC_TRY(ctx_upload(c, L.sol_node, L.n, &i32)); r->lu.sol_node = i32;
+        r->lu.l_nlevels = L.l_nlevels;
+        r->lu.u_nlevels = L.u_nlevels;
+        r->l_level_ptr.assign(L.l_level_ptr, L.l_level_ptr + L.l_nlevels + 1);
+        r->u_level_ptr.assign(L.u_level_ptr, L.u_level_ptr + L.u_nlevels + 1);
+        r->lu.l_level_ptr = r->l_level_ptr.data();
+        r->lu.u_level_ptr = r->u_level_ptr.data();
+        if (L.l_level_lanes) {
+            r->l_lanes.assign(L.l_level_lanes, L.l_level_lanes + L.l_nlevels);
+            r->lu.l_level_lanes = r->l_lanes.data();
+        }
+        if (L.u_level_lanes) {
+            r->u_lanes.assign(L.u_level_lanes, L.u_level_lanes + L.u_nlevels);
+            r->lu.u_level_lanes = r->u_lanes.data();
+        }
+        const int32_t h = L.head;
+        OEC_TRY(ctx_upload(c, L.l_rows, h, &i32)); r->lu.l_rows = i32;
+        OEC_TRY(ctx_upload(c, L.l_ptr, (size_t)h + 1, &i32)); r->lu.l_ptr = i32;
+        const int32_t lnnz = L.l_ptr ? L.l_ptr[h] : 0, unnz = L.u_ptr ? L.u_ptr[h] : 0;
+        OEC_TRY(ctx_upload(c, L.l_idx, lnnz, &i32)); r->lu.l_idx = i32;
+        OEC_TRY(ctx_upload(c, L.l_val, lnnz, &f64)); r->lu.l_val = f64;
+        OEC_TRY(ctx_upload(c, L.u_rows, h, &i32)); r->lu.u_rows = i32;
+        OEC_TRY(ctx_upload(c, L.u_ptr, (size_t)h + 1, &i32)); r->lu.u_ptr = i32;
+        OEC_TRY(ctx_upload(c, L.u_idx, unnz, &i32)); r->lu.u_idx = i32;
+        OEC_TRY(ctx_upload(c, L.u_val, unnz, &f64)); r->lu.u_val = f64;
+        OEC_TRY(ctx_upload(c, L.u_diag, h, &f64)); r->lu.u_diag = f64;
+        if (m > 0) {
+            const int32_t cnnz = L.lc_ptr[m];
+            OEC_TRY(ctx_upload(c, L.lc_ptr, (size_t)m + 1, &i32)); r->lu.lc_ptr = i32;
+            OEC_TRY(ctx_upload(c, L.lc_idx, cnnz, &i32)); r->lu.lc_idx = i32;
+            OEC_TRY(ctx_upload(c, L.lc_val, cnnz, &f64)); r->lu.lc_val = f64;
+            OEC_TRY(ctx_upload(c, L.tl_inv, (size_t)m * m, &f64)); r->lu.tl_inv = f64;
+            OEC_TRY(ctx_upload(c, L.tu_inv, (size_t)m * m, &f64)); r->lu.tu_inv = f64;
+        }
+        OEC_TRY(ctx_array(c, (size_t)L.n + m + 1, &r->lu_work));
     }
-    if (L.u_level_lanes) {
-        r->u_lanes.assign(L.u_level_lanes, L.u_level_lanes + L.u_nlevels);
-        r->lu.u_level_lanes = r->u_lanes.data();
-    }
-    const int32_t h = L.head;
-    OEC_TRY(ctx_upload(c, L.l_rows, h, &i32)); r->lu.l_rows = i32;
-    OEC_TRY(ctx_upload(c, L.l_ptr, (size_t)h + 1, &i32)); r->lu.l_ptr = i32;
-    const int32_t lnnz = L.l_ptr ? L.l_ptr[h] : 0, unnz = L.u_ptr ? L.u_ptr[h] : 0;
-    OEC_TRY(ctx_upload(c, L.l_idx, lnnz, &i32)); r->lu.l_idx = i32;
-    OEC_TRY(ctx_upload(c, L.l_val, lnnz, &f64)); r->lu.l_val = f64;
-    OEC_TRY(ctx_upload(c, L.u_rows, h, &i32)); r->lu.u_rows = i32;
-    OEC_TRY(ctx_upload(c, L.u_ptr, (size_t)h + 1, &i32)); r->lu.u_ptr = i32;
-    OEC_TRY(ctx_upload(c, L.u_idx, unnz, &i32)); r->lu.u_idx = i32;
-    OEC_TRY(ctx_upload(c, L.u_val, unnz, &f64)); r->lu.u_val = f64;
-    OEC_TRY(ctx_upload(c, L.u_diag, h, &f64)); r->lu.u_diag = f64;
-    if (m > 0) {
-        const int32_t cnnz = L.lc_ptr[m];
-        OEC_TRY(ctx_upload(c, L.lc_ptr, (size_t)m + 1, &i32)); r->lu.lc_ptr = i32;
-        OEC_TRY(ctx_upload(c, L.lc_idx, cnnz, &i32)); r->lu.lc_idx = i32;
-        OEC_TRY(ctx_upload(c, L.lc_val, cnnz, &f64)); r->lu.lc_val = f64;
-        OEC_TRY(ctx_upload(c, L.tl_inv, (size_t)m * m, &f64)); r->lu.tl_inv = f64;
-        OEC_TRY(ctx_upload(c, L.tu_inv, (size_t)m * m, &f64)); r->lu.tu_inv = f64;
-    }
-    OEC_TRY(ctx_array(c, (size_t)L.n + m + 1, &r->lu_work));
     const int32_t enz = d->e_ptr[2 * G];
     OEC_TRY(ctx_upload(c, d->e_ptr, 2 * (size_t)G + 1, &r->e_ptr));
     OEC_TRY(ctx_upload(c, d->e_idx, enz, &r->e_idx));

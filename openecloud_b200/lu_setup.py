@@ -9,6 +9,7 @@ imports numpy, scipy and the library's ctypes binding only, so a host that
 drives the library through its context/run handles needs nothing else.
 """
 import ctypes
+import threading
 
 import numpy as np
 import scipy.linalg.lapack as lapack
@@ -26,7 +27,7 @@ class LU_t(ctypes.Structure):
                 ("l_nlevels", ctypes.c_int32), ("l_level_ptr", _P), ("l_rows", _P),
                 ("l_ptr", _P), ("l_idx", _P), ("l_val", _P), ("lc_ptr", _P), ("lc_idx", _P), ("lc_val", _P),
                 ("tl_inv", _P), ("u_nlevels", ctypes.c_int32), ("u_level_ptr", _P), ("u_rows", _P),
-                ("u_ptr", _P), ("u_idx", _P), ("u_val", _P), ("u_diag", _P), ("tu_inv", _P),
+                ("u_ptr", _P), ("u_idx", _P), ("u_val", _P), ("u_diag", _P), ("nd", _P), ("tu_inv", _P),
                 ("head_path", ctypes.c_int32), ("l_level_lanes", _P), ("u_level_lanes", _P)]
 
 
@@ -135,12 +136,30 @@ def assemble(gridObj):
     return a, meps, st, inside
 
 
+class LazyLU:
+    """SuperLU's factor of A with the reference's options
+    (poissonSolver.pyx:59), computed at the first use of one of its
+    attributes: the solve on nested-dissection fronts does not need it."""
+
+    def __init__(self, a):
+        self._a, self._lu, self._lock = a, None, threading.Lock()
+
+    def __getattr__(self, name):
+        if name.startswith("_"):
+            raise AttributeError(name)
+        with self._lock:
+            if self._lu is None:
+                self._lu = spspl.splu(self._a, permc_spec='MMD_AT_PLUS_A', diag_pivot_thresh=0.1)
+        return getattr(self._lu, name)
+
+
 def factor(gridObj):
     """(A, meps, S, inside nodes, SuperLU factor of A with the reference's
-    options, phiToEAtGridPoints) for a grid (poissonSolver.pyx:33-67)."""
+    options (computed on first use), phiToEAtGridPoints) for a grid
+    (poissonSolver.pyx:33-67)."""
     npn = gridObj.getNpExt()
     a, meps, st, inside = assemble(gridObj)
-    lu = spspl.splu(a, permc_spec='MMD_AT_PLUS_A', diag_pivot_thresh=0.1)
+    lu = LazyLU(a)
     phi_to_e = gridObj.getEdgeToNode().dot(spsp.diags(gridObj.getDsi(), 0, (2 * npn, 2 * npn)).dot(st.transpose()))
     return a, meps, st, inside, lu, phi_to_e
 
@@ -202,6 +221,15 @@ def lu_host_arrays(lu, inside, n_nodes, tail=None, inverses=True):
         else:
             a["TL"], a["TU"] = TL, TU
     return a
+
+
+def nd_lu_struct(a, nd):
+    """An LU_t that solves on the fronts of `nd` (an Nd_t the caller keeps)
+    over the arrays `a` of nd_setup.nd_host_arrays."""
+    s = LU_t()
+    s.n, s.head, s.n_nodes = a["n"], a["n"], a["n_nodes"]
+    s.nd = ctypes.addressof(nd)
+    return s
 
 
 def lu_struct(a, ptr):

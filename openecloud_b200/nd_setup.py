@@ -1,0 +1,339 @@
+"""Host-side setup of the nested-dissection Poisson solve, numpy only.
+
+A = S diag(eps0 dsi dst~) S^T over the inside nodes (poissonSolver.pyx:41-58)
+is symmetric and couples grid neighbours only.  The unknowns are split by
+grid lines into a binary tree (oec_nd_dissect); runs of consecutive depths of
+that tree are taken together as the levels of fronts.  A front has s pivots (its
+separators, or the whole set at the bottom) and b boundary unknowns (the
+neighbours of everything below it, pivots of fronts above).  Eliminating level
+by level from the bottom, with F the front's matrix after its children,
+
+    F = [[A11, A21^T], [A21, A22]],   X = A11^-1,   G = A21 X,
+
+the Schur complement A22 - G A21^T goes to the parent.  The device keeps X and G
+of every front: forward, a front sums the updates u of its children into v, and
+y = X v1, u = v2 - G v1; backward, x1 = y - G^T x2.  Both are products of dense
+blocks with a vector, so a solve takes two passes over the levels with no
+dependent chain inside one.
+"""
+import ctypes
+
+import numpy as np
+
+from . import _lib
+
+MAX_LEVELS = 16       # oec_nd_t's array of levels
+MAX_FRONT = 6144      # pivots or boundary unknowns of one front (the device keeps them in shared memory)
+WARP_FRONT = 256      # fronts of at most this many inputs may be taken by one warp each
+LEAF = 12             # unknowns below which a set is not split
+
+
+class NdLevel_t(ctypes.Structure):
+    _fields_ = [(k, ctypes.c_int32) for k in ("fwd_tile", "fwd_tiles", "fwd_width", "bwd_tile", "bwd_tiles",
+                                              "bwd_width", "has_children", "pad")]
+
+
+class Nd_t(ctypes.Structure):
+    _P = ctypes.c_void_p
+    _fields_ = [("n", ctypes.c_int32), ("n_nodes", ctypes.c_int32), ("n_bnd", ctypes.c_int32),
+                ("n_outside", ctypes.c_int32), ("n_levels", ctypes.c_int32), ("max_front", ctypes.c_int32),
+                ("n_fronts", ctypes.c_int32), ("n_tiles", ctypes.c_int32), ("n_mat", ctypes.c_int64),
+                ("level", NdLevel_t * MAX_LEVELS), ("fronts", _P), ("tiles", _P), ("piv_node", _P),
+                ("piv_src", _P), ("bnd_node", _P), ("bnd_src", _P), ("outside", _P), ("mat", _P)]
+
+
+FRONT = np.dtype([("s", np.int32), ("b", np.int32), ("piv0", np.int32), ("bnd0", np.int32), ("ldf", np.int32),
+                  ("ldb", np.int32), ("mf", np.int64), ("mb", np.int64)], align=True)
+
+_lib.OTHER_DECLARED.update({"oec_nd_dissect"})
+
+
+def _declare():
+    L = _lib.lib()
+    if not getattr(L, "_nd_declared", False):
+        P = ctypes.c_void_p
+        L.oec_nd_dissect.restype = ctypes.c_int
+        L.oec_nd_dissect.argtypes = [ctypes.c_int64, P, P, ctypes.c_int32, ctypes.c_int32, P]
+        L._nd_declared = True
+    return L
+
+
+def _ptr(a):
+    return a.ctypes.data_as(ctypes.c_void_p)
+
+
+def dissect(ix, iy, max_depth, leaf=LEAF):
+    """Tree node (root 1, children 2h and 2h + 1) of every unknown."""
+    ix, iy = np.ascontiguousarray(ix, np.int32), np.ascontiguousarray(iy, np.int32)
+    out = np.empty(ix.size, np.int64)
+    rc = _declare().oec_nd_dissect(ix.size, _ptr(ix), _ptr(iy), int(max_depth), int(leaf), _ptr(out))
+    if rc:
+        raise _lib.OecError("oec_nd_dissect", rc)
+    return out
+
+
+# Model of a solve's time by which the levels are chosen (B200): a pass over
+# one level costs its dependent loads and a grid barrier, every front its share
+# of a warp's latency, and the blocks their bytes.
+PHASE_US, FRONT_US, GBS = 3.5, 1.0e-3, 6000.0
+
+
+def choose_levels(hid, dep, w, v, n):
+    """Depths [d_0 = 0, d_1, ...] at which the levels start: level k takes the
+    tree's depths d_k .. d_k+1 - 1, the last one everything from there down.
+    Minimises the modelled time over all choices.  (w, v) are the coupled
+    pairs of unknowns."""
+    top = int(dep.max())
+    size, bnd = [], []
+    for d in range(top + 1):
+        anc = np.where(dep >= d, hid >> np.maximum(dep - d, 0), 0)
+        size.append(np.bincount(anc[anc > 0] - (1 << d), minlength=1 << d))
+        m = (anc[w] > 0) & (anc[v] != anc[w])
+        key = np.unique(anc[w][m] * np.int64(n) + v[m])
+        bnd.append(np.bincount(key // n - (1 << d), minlength=1 << d))
+    end = top + 1
+    best = {end: (0.0, [], 0)}
+    for d in range(end - 1, -1, -1):
+        cand = None
+        for d2 in range(d + 1, end + 1):
+            if best[d2] is None or best[d2][2] + 1 > MAX_LEVELS:
+                continue
+            s = size[d] if d2 == end else size[d] - size[d2].reshape(1 << d, -1).sum(1)
+            b = bnd[d]
+            if s.max() > MAX_FRONT or b.max() > MAX_FRONT:
+                continue
+            s = s.astype(np.float64)
+            t = (1 if d == 0 else 2) * (PHASE_US + FRONT_US * np.count_nonzero(s)) + \
+                8e-3 * float((s * (s + 2.0 * b)).sum()) / GBS + best[d2][0]
+            if cand is None or t < cand[0]:
+                cand = (t, [d] + best[d2][1], best[d2][2] + 1)
+        best[d] = cand
+    return None if best[0] is None else best[0][1]
+
+
+def _width(fronts_out, n_in, ctas):
+    """Outputs per tile of a level: 0 (a warp per front) when the fronts are
+    many and small, else the widest of 64 .. 8 that still gives every CTA a
+    tile."""
+    if n_in <= WARP_FRONT and fronts_out.size >= 4 * ctas:
+        return 0
+    for w in (64, 32, 16):
+        if int((-(-fronts_out // w)).sum()) >= 2 * ctas:
+            return w
+    return 8
+
+
+def nd_host_arrays(a, inside, nx, n_nodes, ctas=296):
+    """oec_nd_t's arrays for the CSC matrix `a` over the nodes `inside` of an
+    extended grid nx nodes wide, or None when A is not a matrix of this form
+    (couplings beyond grid neighbours, not symmetric, a singular front): the
+    level-scheduled factors take it, or refuse it."""
+    n = int(a.shape[0])
+    inside = np.asarray(inside, np.int64)
+    coo = a.tocoo()
+    r, c, val = coo.row.astype(np.int64), coo.col.astype(np.int64), coo.data
+    dist = np.abs(inside[r] - inside[c])
+    if n < 1 or 4 * n > 2 ** 31 - 1 or np.any((dist != 0) & (dist != 1) & (dist != nx)) or \
+            not np.all(np.isfinite(val)) or abs(a - a.T).max() > 0.0:
+        return None
+    off = r != c
+    w, v = r[off], c[off]
+    ix, iy = inside % nx, inside // nx
+    depth = max(0, int(np.ceil(np.log2(max(n, 2) / LEAF))))
+    hid = dissect(ix, iy, depth)
+    dep = np.frexp(hid.astype(np.float64))[1].astype(np.int64) - 1
+    cuts = choose_levels(hid, dep, w, v, n)
+    if cuts is None:
+        return None
+    K = len(cuts)
+    level = np.searchsorted(cuts, dep, side="right") - 1
+    heap = hid >> (dep - np.asarray(cuts)[level])     # tree node of the unknown's front
+    # fronts: level by level from the root, by tree node inside a level
+    key = level * (np.int64(1) << 42) + heap
+    order = np.lexsort((np.arange(n), key))           # unknowns by (front, node)
+    ukey, first, s = np.unique(key[order], return_index=True, return_counts=True)
+    front = np.empty(n, np.int64)
+    front[order] = np.repeat(np.arange(ukey.size), s)
+    pos = np.empty(n, np.int64)
+    pos[order] = np.arange(n)                         # place of an unknown among all pivots
+    flevel = (ukey >> 42).astype(np.int64)
+    fheap = ukey & ((np.int64(1) << 42) - 1)
+    nf = ukey.size
+    # boundary of every front: the neighbours outside of all unknowns below it
+    bkeys = []
+    for k in range(K):
+        d = cuts[k]
+        anc = np.where(dep >= d, hid >> np.maximum(dep - d, 0), 0)
+        m = (anc[w] > 0) & (anc[v] != anc[w])
+        u = np.unique(anc[w][m] * np.int64(n) + v[m])
+        f = np.searchsorted(ukey, k * (np.int64(1) << 42) + u // n)
+        bkeys.append(f * np.int64(n) + u % n)
+    bkey = np.concatenate(bkeys)                      # (front, unknown), ascending
+    bfront, bunk = bkey // n, bkey % n
+    b = np.bincount(bfront, minlength=nf)
+    bnd0 = np.concatenate([[0], np.cumsum(b)])
+    piv0 = np.concatenate([[0], np.cumsum(s)])
+    # parent front (a tree node without unknowns of its own has no front: its children go further up)
+    parent = np.full(nf, -1, np.int64)
+    for k in range(1, K):
+        f = np.nonzero(flevel == k)[0]
+        for up in range(k - 1, -1, -1):
+            f = f[parent[f] < 0]
+            cand = up * (np.int64(1) << 42) + (fheap[f] >> (cuts[k] - cuts[up]))
+            q = np.minimum(np.searchsorted(ukey, cand), nf - 1)
+            hit = ukey[q] == cand
+            parent[f[hit]] = q[hit]
+
+    def local(f, unk):
+        """Index of unknown `unk` in front f's vector [pivots, boundary]."""
+        q = np.searchsorted(bkey, f * np.int64(n) + unk)
+        q = np.minimum(q, bkey.size - 1) if bkey.size else q
+        return np.where(front[unk] == f, pos[unk] - piv0[f], s[f] + q - bnd0[f])
+
+    # contributions: entry e of the children's updates goes to the parent's entry
+    tgt_front = parent[bfront]
+    tgt = local(tgt_front, bunk) if bkey.size else np.zeros(0, np.int64)
+    is_piv = tgt < s[tgt_front] if bkey.size else np.zeros(0, bool)
+    slot_of = np.where(is_piv, piv0[tgt_front] + tgt, n + bnd0[tgt_front] + tgt - s[tgt_front])
+    src = np.full((n + bkey.size, 4), -1, np.int32)
+    e_order = np.argsort(slot_of, kind="stable")
+    so = slot_of[e_order]
+    rank = np.arange(so.size) - np.searchsorted(so, so)
+    if rank.size and rank.max() > 3:
+        return None
+    src[so, rank] = e_order
+    # the blocks
+    ldf, ldb = (s + b + 1) // 2 * 2, (s + 1) // 2 * 2
+    mf = np.concatenate([[0], np.cumsum(s * ldf + b * ldb)])
+    mat = np.zeros(int(mf[-1]))
+    own = np.where(level[r] >= level[c], front[r], front[c])
+    li, lj = local(own, r), local(own, c)
+    by_front = np.argsort(own, kind="stable")
+    own_ptr = np.searchsorted(own[by_front], np.arange(nf + 1))
+    kids = np.argsort(parent, kind="stable")
+    kid_ptr = np.searchsorted(parent[kids], np.arange(nf + 1))
+    schur = {}
+
+    def eliminate(fs):
+        """Fronts fs (of one level, similar size): their blocks into `mat`,
+        their Schur complements into `schur`."""
+        S, B = int(s[fs].max()), int(b[fs].max())
+        T = S + B
+        idx, vals = [], []
+        for k, f in enumerate(fs):
+            e = by_front[own_ptr[f]:own_ptr[f + 1]]
+            i, j = li[e], lj[e]
+            i, j = np.where(i < s[f], i, i - s[f] + S), np.where(j < s[f], j, j - s[f] + S)
+            idx.append((k * T + i) * T + j)
+            vals.append(val[e])
+            for ch in kids[kid_ptr[f]:kid_ptr[f + 1]]:
+                t = tgt[bnd0[ch]:bnd0[ch + 1]]
+                t = np.where(t < s[f], t, t - s[f] + S)
+                idx.append(((k * T + t)[:, None] * T + t).ravel())
+                vals.append(schur.pop(int(ch)).ravel())
+        F = np.bincount(np.concatenate(idx), weights=np.concatenate(vals), minlength=fs.size * T * T)
+        F = F.reshape(fs.size, T, T)
+        A11 = F[:, :S, :S]
+        for k, f in enumerate(fs):
+            A11[k, np.arange(s[f], S), np.arange(s[f], S)] = 1.0
+        X = np.linalg.inv(A11)  # raises LinAlgError on a singular block
+        X = 0.5 * (X + X.transpose(0, 2, 1))
+        A21 = F[:, S:, :S]
+        G = A21 @ X
+        C = F[:, S:, S:] - G @ A21.transpose(0, 2, 1) if B else None
+        for k, f in enumerate(fs):
+            sf, bf, o = int(s[f]), int(b[f]), int(mf[f])
+            fw = mat[o:o + sf * ldf[f]].reshape(sf, ldf[f])
+            fw[:, :sf] = X[k, :sf, :sf]
+            if bf:
+                fw[:, sf:sf + bf] = G[k, :bf, :sf].T
+                o += sf * int(ldf[f])
+                mat[o:o + bf * ldb[f]].reshape(bf, ldb[f])[:, :sf] = G[k, :bf, :sf]
+                schur[int(f)] = np.ascontiguousarray(C[k, :bf, :bf])
+
+    # one after another: BLAS threads the large fronts by itself
+    for k in range(K - 1, -1, -1):
+        fs = np.nonzero(flevel == k)[0]
+        fs = fs[np.lexsort((b[fs], s[fs]))]
+        # chunks of up to ~4 M matrix entries
+        chunk = np.cumsum((s[fs] + b[fs]) ** 2) // 4_000_000
+        for part in np.split(fs, np.nonzero(np.diff(chunk))[0] + 1):
+            try:
+                eliminate(part)
+            except np.linalg.LinAlgError:
+                return None
+    out = {"n": n, "n_nodes": int(n_nodes), "n_bnd": int(bkey.size), "n_levels": K, "n_fronts": nf,
+           "max_front": int(max(s.max(), b.max())), "cuts": list(cuts), "level_of_front": flevel}
+    fr = np.zeros(nf, FRONT)
+    fr["s"], fr["b"], fr["piv0"], fr["bnd0"] = s, b, piv0[:-1], bnd0[:-1]
+    fr["ldf"], fr["ldb"], fr["mf"], fr["mb"] = ldf, ldb, mf[:-1], mf[:-1] + s * ldf
+    out["fronts"] = fr
+    mask = np.ones(int(n_nodes), bool)
+    mask[inside] = False
+    out["outside"] = np.nonzero(mask)[0].astype(np.int32)
+    out["piv_node"] = inside[order].astype(np.int32)
+    out["bnd_node"] = inside[bunk].astype(np.int32)
+    out["piv_src"], out["bnd_src"] = np.ascontiguousarray(src[:n]), np.ascontiguousarray(src[n:])
+    out["mat"] = mat
+    # tiles: (front, first output) per CTA, or (front, 0) per warp
+    tiles, lv = [], []
+    count = 0
+    for k in range(K):
+        fs = np.nonzero(flevel == k)[0]
+        rec = {"has_children": int(np.any(np.isin(parent, fs)))}
+        for tag, outs, ins in (("fwd", s[fs] + b[fs], s[fs]), ("bwd", s[fs] if k else 0 * s[fs], b[fs])):
+            wd = _width(outs, int(ins.max()) if ins.size else 0, ctas)
+            per = np.where(outs > 0, 1, 0) if wd == 0 else -(-outs // wd)
+            t = np.zeros((int(per.sum()), 2), np.int32)
+            t[:, 0] = np.repeat(fs, per)
+            t[:, 1] = (np.arange(t.shape[0]) - np.repeat(np.cumsum(per) - per, per)) * wd
+            rec.update({tag + "_tile": count, tag + "_tiles": t.shape[0], tag + "_width": wd})
+            count += t.shape[0]
+            tiles.append(t)
+        lv.append(rec)
+    out["tiles"] = np.ascontiguousarray(np.concatenate(tiles))
+    out["level"] = lv
+    return out
+
+
+def nd_struct(a, ptr):
+    """An Nd_t over the arrays of nd_host_arrays; ptr(name) gives the address
+    of array `name` (host or device copy)."""
+    t = Nd_t()
+    for k in ("n", "n_nodes", "n_bnd", "n_levels", "max_front", "n_fronts"):
+        setattr(t, k, a[k])
+    t.n_outside, t.n_tiles, t.n_mat = a["outside"].size, a["tiles"].shape[0], a["mat"].size
+    for k, rec in enumerate(a["level"]):
+        for name, x in rec.items():
+            setattr(t.level[k], name, x)
+    for name in ("fronts", "tiles", "piv_node", "piv_src", "bnd_node", "bnd_src", "outside", "mat"):
+        setattr(t, name, ptr(name))
+    return t
+
+
+def nd_solve_host(a, q):
+    """The device's solve restated with numpy: phi on all nodes."""
+    n = a["n"]
+    y, u, phi = np.zeros(n), np.zeros(a["n_bnd"] + 1), np.zeros(a["n_nodes"])
+    fr, mat = a["fronts"], a["mat"]
+
+    def gathered(src):
+        return u[src].sum(1)  # -1 is the zero behind the last update
+
+    for k in range(a["n_levels"] - 1, -1, -1):
+        for f in np.nonzero(a["level_of_front"] == k)[0]:
+            s, b, p0, b0 = (int(fr[f][x]) for x in ("s", "b", "piv0", "bnd0"))
+            v1 = q[a["piv_node"][p0:p0 + s]] + gathered(a["piv_src"][p0:p0 + s])
+            m = mat[fr[f]["mf"]:fr[f]["mf"] + s * fr[f]["ldf"]].reshape(s, -1)[:, :s + b]
+            o = v1 @ m
+            y[p0:p0 + s] = o[:s]
+            u[b0:b0 + b] = gathered(a["bnd_src"][b0:b0 + b]) - o[s:]
+    for k in range(a["n_levels"]):
+        for f in np.nonzero(a["level_of_front"] == k)[0]:
+            s, b, p0, b0 = (int(fr[f][x]) for x in ("s", "b", "piv0", "bnd0"))
+            x1 = y[p0:p0 + s].copy()
+            if b:
+                m = mat[fr[f]["mb"]:fr[f]["mb"] + b * fr[f]["ldb"]].reshape(b, -1)[:, :s]
+                x1 -= phi[a["bnd_node"][b0:b0 + b]] @ m
+            phi[a["piv_node"][p0:p0 + s]] = x1
+    return phi

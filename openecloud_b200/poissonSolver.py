@@ -30,7 +30,8 @@ from . import _lib
 from . import device as D
 from .constants import epsilon_0
 from .lu_setup import (LU_t, _level_lists, _levels, _np_ptr, assemble, choose_tail, factor,  # noqa: F401
-                       level_lanes, lu_host_arrays, lu_struct)
+                       level_lanes, lu_host_arrays, lu_struct, nd_lu_struct)
+from .nd_setup import nd_host_arrays, nd_struct
 
 
 class Stencil_t(ctypes.Structure):
@@ -363,11 +364,34 @@ class PoissonSolver:
 
     # -------------------------------------------------------------- setup
     def _device_setup(self, tail):
+        """Uploads what the direct solve runs on: the nested-dissection fronts
+        (nd_setup.nd_host_arrays), or with a `tail` given (and for a matrix
+        that has no such fronts) the head/tail form of SuperLU's factors."""
+        E = self.phiToEAtGridPoints.tocsr()
+        E.sort_indices()
+        self._keep = k = {}
+        k["e_ptr"], k["e_idx"] = D.to_device(E.indptr, torch.int32), D.to_device(E.indices, torch.int32)
+        k["e_val"] = D.to_device(E.data, torch.float64)
+        nd = None if tail is not None else \
+            nd_host_arrays(self.systemMatrix, self.insidePointsInd, self.gridObj.getNxExt(), self.n_nodes)
+        if nd is None:
+            self._factor_setup(tail)
+            return
+        for name in ("tiles", "piv_node", "piv_src", "bnd_node", "bnd_src", "outside"):
+            k[name] = D.to_device(nd[name], torch.int32)
+        k["fronts"] = D.to_device(nd["fronts"].view(np.uint8), torch.uint8)
+        k["mat"] = D.to_device(nd["mat"], torch.float64)
+        self._nd_t = nd_struct(nd, lambda name: D.ptr(k[name]))
+        self._lu_t = nd_lu_struct(nd, self._nd_t)
+        self._work = D.zeros(nd["n"] + nd["n_bnd"] + 1, torch.float64)
+        self.tail = 0
+        self.levels = (nd["n_levels"], nd["n_levels"])
+
+    def _factor_setup(self, tail):
         """Uploads the head/tail form of the factors (lu_setup.lu_host_arrays);
         the tail blocks are inverted on the device."""
         a = lu_host_arrays(self.ludecom, self.insidePointsInd, self.n_nodes, tail, inverses=False)
         self.tail = m = a["tail"]
-        self._keep = {}
         k = self._keep
         for name in ("rhs_node", "sol_src", "sol_node", "l_rows", "l_ptr", "l_idx", "u_rows", "u_ptr", "u_idx",
                      "lc_ptr", "lc_idx"):
@@ -388,10 +412,6 @@ class PoissonSolver:
         self._l_level_lanes, self._u_level_lanes = a["l_level_lanes"], a["u_level_lanes"]
         self._lu_t = lu_struct(a, lambda name: D.ptr(k.get(name)))
         self._work = D.zeros(a["n"] + m + 1, torch.float64)
-        E = self.phiToEAtGridPoints.tocsr()
-        E.sort_indices()
-        k["e_ptr"], k["e_idx"] = D.to_device(E.indptr, torch.int32), D.to_device(E.indices, torch.int32)
-        k["e_val"] = D.to_device(E.data, torch.float64)
         self.levels = (a["l_nlevels"], a["u_nlevels"])
 
     # -------------------------------------------------------------- solve

@@ -26,7 +26,8 @@ from .beam import LHCBeam, LHCBeamEndless
 from .constants import elementary_charge, m_e
 from .furman import Furman_t, furman_params, furman_struct
 from .grid import Grid
-from .lu_setup import LU_t, factor, lu_host_arrays, lu_struct
+from .lu_setup import LU_t, factor, lu_host_arrays, lu_struct, nd_lu_struct
+from .nd_setup import nd_host_arrays, nd_struct
 
 _P = ctypes.c_void_p
 
@@ -130,8 +131,12 @@ class Run:
         self._keep = keep = {}
         keep["profile"] = np.ascontiguousarray(bm.getTransversalProfile(), np.float64)
         keep["table"] = np.ascontiguousarray(bm.scalarTable(int(n_steps_table)), np.float64)
-        _, _, _, inside, lu, phi_to_e = factor(g)
-        keep["lu"] = a = lu_host_arrays(lu, inside, g.getNpExt(), tail)
+        matrix, _, _, inside, lu, phi_to_e = factor(g)
+        keep["nd"] = nd = None if tail is not None else nd_host_arrays(matrix, inside, g.getNxExt(), g.getNpExt())
+        if nd is None:
+            keep["lu"] = a = lu_host_arrays(lu, inside, g.getNpExt(), tail)
+        else:
+            keep["nd_t"] = nd_struct(nd, lambda name: _ptr(nd[name]))
         E = phi_to_e.tocsr()
         E.sort_indices()
         keep["e_ptr"] = np.ascontiguousarray(E.indptr, np.int32)
@@ -156,7 +161,7 @@ class Run:
         d.emit_seed = int(seed) + 17      # the seed Buildup gives its FurmanEmitter
         d.manage_seed = int(seed)
         d.beam_profile, d.beam_table = _ptr(keep["profile"]), _ptr(keep["table"])
-        d.lu = lu_struct(a, lambda name: _ptr(a.get(name)))
+        d.lu = lu_struct(a, lambda name: _ptr(a.get(name))) if nd is None else nd_lu_struct(nd, keep["nd_t"])
         d.e_ptr, d.e_idx, d.e_val = _ptr(keep["e_ptr"]), _ptr(keep["e_idx"]), _ptr(keep["e_val"])
         h = _P()
         _call("oec_run_create", ctx.handle, ctypes.byref(d), ctypes.byref(h))

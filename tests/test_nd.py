@@ -1,0 +1,86 @@
+"""The direct solve on nested-dissection fronts, against a sparse solve of the
+assembled matrix.
+
+Tolerance: both sides are backward stable up to small factors, so they differ
+by at most about eps times the condition number, which for the 5-point
+operator on nx x ny cells is below nx^2 + ny^2 (times the squared aspect ratio
+of a cell); 16 eps of that."""
+import numpy as np
+import pytest
+import scipy.sparse as spsp
+import scipy.sparse.linalg as spla
+
+# nx, ny, lx, ly, boundType: a single unknown row, one front, several levels, odd and elongated grids
+GRIDS = [(3, 3, 0.04, 0.04, 0), (5, 4, 0.04, 0.03, 0), (33, 25, 0.04, 0.03, 0), (24, 200, 0.02, 0.1, 0),
+         (64, 48, 0.04, 0.04, 1), (131, 97, 0.06, 0.05, 1), (200, 151, 0.09, 0.036, 1)]
+
+
+def _case(p):
+    from openecloud_b200.grid import Grid
+    from openecloud_b200.lu_setup import assemble
+    g = Grid(*p)
+    a, _, _, inside = assemble(g)
+    q = np.zeros(g.getNpExt())
+    q[inside] = np.random.default_rng(p[0]).normal(size=inside.size) * 1e-9
+    r = g.getDx() / g.getDy()
+    tol = 16 * 2.3e-16 * (p[0] ** 2 + p[1] ** 2) * max(r, 1 / r) ** 2
+    phi = np.zeros(q.size)
+    phi[inside] = spla.spsolve(a.tocsc(), q[inside])
+    return g, a, inside, q, phi, tol
+
+
+@pytest.mark.parametrize("levels", ["model", "many"])
+@pytest.mark.parametrize("p", GRIDS)
+def test_fronts_on_the_host(p, levels, monkeypatch):
+    """The setup's fronts, replayed with numpy, solve the matrix; with a phase
+    that costs nothing the tree is cut at (nearly) every depth."""
+    from openecloud_b200 import nd_setup
+    if levels == "many":
+        monkeypatch.setattr(nd_setup, "PHASE_US", 0.0)
+        monkeypatch.setattr(nd_setup, "FRONT_US", 0.0)
+    g, a, inside, q, phi, tol = _case(p)
+    h = nd_setup.nd_host_arrays(a, inside, g.getNxExt(), g.getNpExt())
+    x = nd_setup.nd_solve_host(h, q)
+    assert np.linalg.norm(x - phi) <= tol * np.linalg.norm(phi)
+    assert h["piv_node"].size == np.unique(h["piv_node"]).size == inside.size
+    if levels == "many" and inside.size > 1000:
+        assert h["n_levels"] >= 5
+
+
+def test_other_matrices_are_left_to_the_factors():
+    """A matrix that couples other than grid neighbours, is not symmetric or
+    has a singular front gets no fronts."""
+    from openecloud_b200 import nd_setup
+    g, a, inside, *_ = _case(GRIDS[2])
+    args = (inside, g.getNxExt(), g.getNpExt())
+    far = a.tolil()
+    far[0, 40] = far[40, 0] = -1e-12
+    assert nd_setup.nd_host_arrays(far.tocsc(), *args) is None
+    skew = a.tolil()
+    skew[0, 1] = 2 * a[0, 1]
+    assert nd_setup.nd_host_arrays(skew.tocsc(), *args) is None
+    assert nd_setup.nd_host_arrays(spsp.csc_matrix((inside.size, inside.size)), *args) is None
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("levels", ["model", "many"])
+@pytest.mark.parametrize("p", GRIDS + [(402, 301, 0.09, 0.036, 1)])
+def test_fronts_on_the_device(gpu, p, levels, monkeypatch):
+    """One solve per grid and choice of levels (one front, CTA tiles of every
+    width, a warp per front), twice: the same bits, and zero outside."""
+    from openecloud_b200 import nd_setup
+    from openecloud_b200.poissonSolver import PoissonSolver
+    if levels == "many":
+        monkeypatch.setattr(nd_setup, "PHASE_US", 0.0)
+        monkeypatch.setattr(nd_setup, "FRONT_US", 0.0)
+    g, a, inside, q, phi, tol = _case(p)
+    ps = PoissonSolver(g)
+    assert ps._lu_t.nd
+    ps.phi.fill_(3.0)
+    ps.solve(q)
+    x = ps.getPhi()
+    assert np.linalg.norm(x - phi) <= tol * np.linalg.norm(phi)
+    ps.phi.fill_(-1.0)
+    ps.solve(q)
+    assert np.array_equal(ps.getPhi(), x)
+    assert np.all(np.delete(x, inside) == 0.0)
