@@ -5,7 +5,7 @@
 //  pass 1: primary energy and incidence angle, elastic/rediffused/true yields
 //          and the number of secondaries drawn from P_n (:180-229);
 //  scan:   output offsets of each absorbed particle's secondaries;
-//  pass 2: energies (single secondary: elastic/rediffused/true split;
+//  emit:   energies (single secondary: elastic/rediffused/true split;
 //          several: the joint energy split through I_x and P inverses,
 //          :232-278) and cos-law directions about the wall normal (:280-302).
 // Every absorbed particle draws from its own Philox stream, so the emitted
@@ -41,19 +41,50 @@ __device__ __forceinline__ double clip(double x, double lo, double hi) {
     return hi;
 }
 
-__global__ void k_furman_pass1(oec_furman_t f, const double *__restrict__ rows, const double *__restrict__ normals,
-                               const int32_t *n_abs, int cap, const int32_t *__restrict__ ids, uint2 key,
-                               uint32_t step, const int32_t *step_dev, const double *__restrict__ replay,
-                               Rec *__restrict__ rec,
-                               int32_t *__restrict__ nsec, oec_status_t *status) {
+constexpr int kSlots = 10;
+constexpr int kClasses = kSlots * (kSlots + 1) / 2;  // (n, k), k < n: n (n - 1) / 2 + k
+
+// The constants of the inverses of k_furman_emit, by (n, k).
+struct SplitConst {
+    sf::BetaConst beta[kClasses - kSlots];  // k < n - 1: (n - 1) (n - 2) / 2 + k
+    sf::GammaConst gamma[kSlots];           // k = n - 1: n - 1
+    sf::GammaConst gamma1[kSlots];          // P(pSmallN[n-1], .): n - 1
+};
+
+// The blocks behind the first `row_blocks` lay out the constants of one class
+// (n, k) each for the next kernels, beside the rows' work.
+__global__ void __launch_bounds__(128)
+    k_furman_pass1(oec_furman_t f, const double *__restrict__ rows, const double *__restrict__ normals,
+                   const int32_t *n_abs, int cap, const int32_t *__restrict__ ids, uint2 key, uint32_t step,
+                   const int32_t *step_dev, const double *__restrict__ replay, Rec *__restrict__ rec,
+                   int32_t *__restrict__ nsec, oec_status_t *status, int row_blocks, SplitConst *__restrict__ consts) {
+    if ((int)blockIdx.x >= row_blocks) {
+        const int c = blockIdx.x - row_blocks;
+        int n = 1, k;
+        if (c < kClasses) {
+            while (n * (n + 1) / 2 <= c) ++n;
+            k = c - n * (n - 1) / 2;
+        } else {
+            n = k = c - kClasses + 1;
+        }
+        const double P = f.pSmallN[n - 1];
+        if (k == n)  // the blocks behind the classes
+            sf::gamma_const(P, consts->gamma1[n - 1]);
+        else if (k == n - 1)
+            sf::gamma_const(n * P, consts->gamma[n - 1]);
+        else
+            sf::beta_const(P * (n - k - 1), P, consts->beta[(n - 1) * (n - 2) / 2 + k]);
+        return;
+    }
     int na = min(*n_abs, cap);
     const double eFactor = 0.5 * f.particle_mass / 1.602176565e-19;
     int wd = 0, wt = 0;
-    double lfac[11];  // lgamma(j + 1), j <= m <= 10, by the threads that have work
-    if ((int)(blockIdx.x * blockDim.x + threadIdx.x) < na)
-        for (int j = 0; j <= f.m; ++j) lfac[j] = sf::lgam((double)j + 1.0);
+    __shared__ double lfac[11];  // lgamma(j + 1), j <= m <= 10
+    if ((int)(blockIdx.x * blockDim.x) >= na) return;
+    if (threadIdx.x <= f.m) lfac[threadIdx.x] = sf::lgam((double)threadIdx.x + 1.0);
+    __syncthreads();
     int skipped = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < na; i += gridDim.x * blockDim.x) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < na; i += row_blocks * blockDim.x) {
         const double *r = rows + 6 * (int64_t)i;
         const double n0 = normals[2 * i], n1 = normals[2 * i + 1];
         double v0 = sqrt(r[2] * r[2] + r[3] * r[3] + r[4] * r[4]);
@@ -122,116 +153,178 @@ __global__ void k_furman_pass1(oec_furman_t f, const double *__restrict__ rows, 
     if (skipped) atomicAdd(&status->n_emit_skipped, skipped);
 }
 
-// Pass 2a: the costly inverses of the joint energy split of a multi-secondary
-// emission (particleEmitter.pyx:255-266), one thread per (absorbed particle,
-// slot).  For n secondaries slot k < n-1 holds theta_k =
-// asin(sqrt(I^-1_u(P(n-k-1), P))) from draw 1+k and slot n-1 holds
-// y = sqrt(P^-1(nP, u p0)) from draw n: the same draws and the same
-// arithmetic as one thread doing them in sequence, but the n calls run side
-// by side instead of one after the other.
-constexpr int kSlots = 10;
-
-__global__ void k_furman_pass2a(oec_furman_t f, const int32_t *n_abs, int cap, const int32_t *__restrict__ ids,
-                                uint2 key, uint32_t step, const int32_t *step_dev, const double *__restrict__ replay,
-                                const Rec *__restrict__ rec, double *__restrict__ split) {
-    const int na = min(*n_abs, cap);
-    const int total = na * kSlots;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-        const int i = t / kSlots, k = t % kSlots;
-        const Rec R = rec[i];
-        const int n = R.nsec;
-        if (n < 2 || k >= n) continue;
-        const double P = f.pSmallN[n - 1], eps = f.epsN[n - 1];
-        sf::Draws dr{key, ids ? (uint32_t)ids[i] : (uint32_t)i, step + (step_dev ? (uint32_t)*step_dev : 0u),
-                     replay ? replay + (int64_t)i * kDraws : nullptr};
-        dr.d = 1 + k;
-        double v;
-        if (k < n - 1) {
-            v = asin(sqrt(sf::betaincinv(P * (n - k - 1), P, dr.next())));
-        } else {
-            const double p0 = sf::gammainc(n * P, R.e0 / eps);
-            v = sqrt(sf::gammaincinv(n * P, dr.next() * p0));
-        }
-        split[(int64_t)i * kSlots + k] = v;
-    }
+// A secondary's direction: cos-law about the normal (:280-302), draws dr.d and
+// dr.d + 1.  sin(asin u) = u and cos(asin u) = sqrt(1 - u^2).
+__device__ __forceinline__ void put_secondary(const double *r, double n0, double n1, double vs, sf::Draws &dr,
+                                              double *q) {
+    const double sT = dr.next(), cT = sqrt((1. - sT) * (1. + sT));
+    double sP, cP;
+    sincos(dr.next() * sf::kPi * 2., &sP, &cP);
+    const double t1 = cT * n0 - sT * n1;
+    const double t2 = sT * n0 + cT * n1;
+    q[0] = r[0];
+    q[1] = r[1];
+    q[2] = vs * ((cP + n0 * n0 * (1 - cP)) * t1 + n0 * n1 * (1 - cP) * t2);
+    q[3] = vs * ((cP + n1 * n1 * (1 - cP)) * t2 + n0 * n1 * (1 - cP) * t1);
+    q[4] = vs * (-sP * n1 * t1 + sP * n0 * t2);
+    q[5] = r[5];
 }
 
-__global__ void k_furman_pass2(oec_furman_t f, const double *__restrict__ rows, const double *__restrict__ normals,
-                               const int32_t *n_abs, int cap, const int32_t *__restrict__ ids, uint2 key,
-                               uint32_t step, const int32_t *step_dev, const double *__restrict__ replay,
-                               const Rec *__restrict__ rec, const double *__restrict__ split,
-                               const int32_t *__restrict__ offset, double *__restrict__ out, int out_cap,
-                               oec_status_t *status) {
-    int na = min(*n_abs, cap);
-    if (na <= 0) return;
+// Energies and directions of all secondaries (particleEmitter.pyx:232-302).
+// A lone one splits into elastic, rediffused and true.  n > 1 share the energy:
+// slot k < n-1 takes B_k = I^-1_u(P(n-k-1), P) from draw 1+k, slot n-1 takes y =
+// sqrt(P^-1(nP, u p0)) from draw n, and with sin(theta_k)^2 = B_k secondary k
+// gets eps (y cos(theta_k) prod_{t<k} sin(theta_t))^2, the last one without
+// the cosine.
+//
+// The inverses are most of the work.  They differ in their branch and their
+// length by (n, k) above all, and most of a row's kSlots slots are empty, so a
+// CTA takes a chunk of rows, sorts its secondaries by (n, k) in shared memory and
+// works them off in that order, a warp taking the next 32 when it is free: the
+// lanes of a warp run the same branch of the same function, with the
+// constants of (n, k) from pass 1 (specfun.cuh).  Which lane takes which
+// does not enter its value.  106,457 absorbed rows of 200 eV electrons (179,048
+// secondaries) on a B200: 3340 us for a thread per (row, slot) with the plain
+// inverses and a thread per row for the directions, 132 us this way; 250 secondaries
+// (one buildup step): 40 us, the latency of one inverse.
+constexpr int kSplitT = 256, kSplitRows = 1024;
+
+struct SplitShared {
+    SplitConst c;
+    int count[kClasses + 1];                // secondaries, then the place after the last one put
+    int next[2];                            // secondaries handed out to the warps, per phase
+    unsigned char nsec[kSplitRows];
+    unsigned task[kSplitRows * kSlots];     // row in the chunk | n << 16 | k << 24
+};
+
+// The next 32 secondaries for this warp; this lane's one, or -1.  False when
+// none are left.
+__device__ __forceinline__ bool next_task(int *next, int total, int *t) {
+    int b = 0;
+    if ((threadIdx.x & 31) == 0) b = atomicAdd(next, 32);
+    b = __shfl_sync(kFullMask, b, 0);
+    *t = b + (int)(threadIdx.x & 31);
+    if (*t >= total) *t = -1;
+    return b < total;
+}
+
+__global__ void __launch_bounds__(kSplitT)
+    k_furman_emit(oec_furman_t f, const double *__restrict__ rows, const double *__restrict__ normals,
+                  const int32_t *n_abs, int cap, const int32_t *__restrict__ ids, uint2 key, uint32_t step,
+                  const int32_t *step_dev, const double *__restrict__ replay, const Rec *__restrict__ rec,
+                  const SplitConst *__restrict__ consts, double *__restrict__ split,
+                  const int32_t *__restrict__ offset, double *__restrict__ out, int out_cap, oec_status_t *status) {
+    extern __shared__ __align__(16) unsigned char split_smem[];
+    SplitShared &sh = *reinterpret_cast<SplitShared *>(split_smem);
+    const int na = min(*n_abs, cap);
+    // rows per chunk: all CTAs busy before the chunks reach full size
+    const int per = (na + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int chunk = min(kSplitRows, max(32, (per + 31) & ~31));
+    if ((int)blockIdx.x * chunk >= na) return;
+    const uint32_t st = step + (step_dev ? (uint32_t)*step_dev : 0u);
+    const int tid = threadIdx.x;
     const double eFactorInv = 1.0 / (0.5 * f.particle_mass / 1.602176565e-19);
     const Rec last = rec[na - 1];
+    static_assert(sizeof(SplitConst) % sizeof(int4) == 0, "copied by 16 bytes");
+    for (int i = tid; i < (int)(sizeof(SplitConst) / sizeof(int4)); i += kSplitT)
+        reinterpret_cast<int4 *>(&sh.c)[i] = __ldg(reinterpret_cast<const int4 *>(consts) + i);
     int dropped = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < na; i += gridDim.x * blockDim.x) {
-        const Rec R = rec[i];
-        const int n = R.nsec;
-        if (n == 0) continue;
-        const double *r = rows + 6 * (int64_t)i;
-        const double n0 = normals[2 * i], n1 = normals[2 * i + 1];
-        sf::Draws dr{key, ids ? (uint32_t)ids[i] : (uint32_t)i, step + (step_dev ? (uint32_t)*step_dev : 0u),
-                     replay ? replay + (int64_t)i * kDraws : nullptr};
-        dr.d = 1;  // draw 0 was the secondary count
-        double eSec[10];
-        const double e0 = R.e0;
-        if (n == 1) {
+    for (int r0 = blockIdx.x * chunk; r0 < na; r0 += gridDim.x * chunk) {
+        const int nrows = min(chunk, na - r0);
+        for (int c = tid; c <= kClasses; c += kSplitT) sh.count[c] = 0;
+        if (tid < 2) sh.next[tid] = 0;
+        __syncthreads();
+        for (int r = tid; r < nrows; r += kSplitT) {
+            const int n = rec[r0 + r].nsec;
+            sh.nsec[r] = (unsigned char)n;
+            for (int k = 0; k < n; ++k) atomicAdd(&sh.count[n * (n - 1) / 2 + k], 1);
+        }
+        __syncthreads();
+        if (tid < 32) {  // exclusive scan of the counts by one warp
+            int carry = 0;
+            for (int c0 = 0; c0 <= kClasses; c0 += 32) {
+                const int c = c0 + tid, v = c < kClasses ? sh.count[c] : 0;
+                int x = v;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(kFullMask, x, o);
+                    if (tid >= o) x += y;
+                }
+                if (c <= kClasses) sh.count[c] = carry + x - v;
+                carry += __shfl_sync(kFullMask, x, 31);
+            }
+        }
+        __syncthreads();
+        const int total = sh.count[kClasses], lone = sh.count[1];  // class 0 comes first
+        __syncthreads();
+        for (int r = tid; r < nrows; r += kSplitT) {
+            const int n = sh.nsec[r];
+            for (int k = 0; k < n; ++k) sh.task[atomicAdd(&sh.count[n * (n - 1) / 2 + k], 1)] = r | n << 16 | k << 24;
+        }
+        __syncthreads();
+        // the inverses; a lone secondary is finished here
+        int t;
+        while (next_task(&sh.next[0], total, &t)) {
+            if (t < 0) continue;
+            const unsigned w = sh.task[t];
+            const int row = r0 + (int)(w & 0xffff), n = (w >> 16) & 0xff, k = w >> 24;
+            sf::Draws dr{key, ids ? (uint32_t)ids[row] : (uint32_t)row, st,
+                         replay ? replay + (int64_t)row * kDraws : nullptr};
+            dr.d = 1 + k;  // draw 0 was the secondary count
+            const double u = dr.next();
+            if (k < n - 1) {
+                split[(int64_t)row * kSlots + k] = sf::betaincinv_t(sh.c.beta[(n - 1) * (n - 2) / 2 + k], sh.c.gamma1[n - 1], u);
+                continue;
+            }
+            const sf::GammaConst &G = sh.c.gamma[n - 1];
+            const double e0 = rec[row].e0;
+            if (n > 1) {
+                split[(int64_t)row * kSlots + k] = sf::gammaincinv_t(G, u * sf::gammainc_of(G, e0 / f.epsN[n - 1]));
+                continue;
+            }
             // compat: the reference reads the split of the LAST absorbed particle
             // of pass 1 (stale loop variables, particleEmitter.pyx:245-246)
-            const Rec &S = f.compat_last ? last : R;
-            double aE = S.dE / S.pN1, aR = S.dR / S.pN1;
-            double u = dr.next();
+            const Rec S = f.compat_last ? last : rec[row];
+            const double aE = S.dE / S.pN1, aR = S.dR / S.pN1;
+            double e;
             if (u < aE) {
-                double sig = f.scaleSigmaE ? f.sigmaE * sqrt(e0 / 300) : f.sigmaE;
-                eSec[0] = e0 - fabs(sig * dr.normal());
-                if (eSec[0] < 0.) eSec[0] = dr.next() * e0;
+                const double sig = f.scaleSigmaE ? f.sigmaE * sqrt(e0 / 300) : f.sigmaE;
+                e = e0 - fabs(sig * dr.normal());
+                if (e < 0.) e = dr.next() * e0;
             } else if (u < aE + aR) {
-                eSec[0] = e0 * pow(dr.next(), 1. / (1. + f.q));
+                e = e0 * pow(dr.next(), 1. / (1. + f.q));
             } else {
-                eSec[0] = f.epsN[0] * sf::gammaincinv(f.pSmallN[0], dr.next() * sf::gammainc(f.pSmallN[0], e0 / f.epsN[0]));
+                e = f.epsN[0] * sf::gammaincinv_t(G, dr.next() * sf::gammainc_of(G, e0 / f.epsN[0]));
             }
-        } else {
-            // theta_k and y from pass 2a (draws 1 .. n)
-            const double *sp = split + (int64_t)i * kSlots;
-            const double eps = f.epsN[n - 1];
-            double th[10];
-            for (int k = 0; k < n - 1; ++k) th[k] = sp[k];
-            const double y = sp[n - 1];
-            dr.d = n + 1;
-            double yk[10];
-            yk[0] = y * cos(th[0]);
-            yk[n - 1] = y;
-            for (int k = 0; k < n - 1; ++k) yk[n - 1] *= sin(th[k]);
-            for (int k = 1; k < n - 1; ++k) {
-                yk[k] = y * cos(th[k]);
-                for (int t = 0; t < k; ++t) yk[k] *= sin(th[t]);
-            }
-            for (int k = 0; k < n; ++k) eSec[k] = eps * (yk[k] * yk[k]);
+            const int o = offset[row];
+            if (o < out_cap)
+                put_secondary(rows + 6 * (int64_t)row, normals[2 * row], normals[2 * row + 1], sqrt(eFactorInv * e), dr,
+                              out + 6 * (int64_t)o);
+            else
+                ++dropped;
         }
-        int o = offset[i];
-        for (int k = 0; k < n; ++k) {
-            double vs = sqrt(eFactorInv * eSec[k]);
-            double thS = asin(dr.next());
-            double cT = cos(thS), sT = sin(thS);
-            double phS = dr.next() * sf::kPi * 2.;
-            double cP = cos(phS), sP = sin(phS);
-            double t1 = cT * n0 - sT * n1;
-            double t2 = sT * n0 + cT * n1;
-            if (o + k >= out_cap) {
+        __syncthreads();
+        // the shared energies and the directions
+        while (next_task(&sh.next[1], total - lone, &t)) {
+            if (t < 0) continue;
+            const unsigned w = sh.task[lone + t];
+            const int row = r0 + (int)(w & 0xffff), n = (w >> 16) & 0xff, k = w >> 24;
+            const int o = offset[row] + k;
+            if (o >= out_cap) {
                 ++dropped;
                 continue;
             }
-            double *q = out + 6 * (int64_t)(o + k);
-            q[0] = r[0];
-            q[1] = r[1];
-            q[2] = vs * ((cP + n0 * n0 * (1 - cP)) * t1 + n0 * n1 * (1 - cP) * t2);
-            q[3] = vs * ((cP + n1 * n1 * (1 - cP)) * t2 + n0 * n1 * (1 - cP) * t1);
-            q[4] = vs * (-sP * n1 * t1 + sP * n0 * t2);
-            q[5] = r[5];
+            const double *B = split + (int64_t)row * kSlots;
+            double e = B[n - 1];
+            for (int j = 0; j < k; ++j) e *= B[j];
+            if (k < n - 1) e *= 1. - B[k];
+            sf::Draws dr{key, ids ? (uint32_t)ids[row] : (uint32_t)row, st,
+                         replay ? replay + (int64_t)row * kDraws : nullptr};
+            dr.d = n + 1 + 2 * k;
+            put_secondary(rows + 6 * (int64_t)row, normals[2 * row], normals[2 * row + 1],
+                          sqrt(eFactorInv * (f.epsN[n - 1] * e)), dr, out + 6 * (int64_t)o);
         }
+        __syncthreads();
     }
     if (dropped) atomicAdd(&status->n_capacity_drop, dropped);
 }
@@ -552,26 +645,35 @@ extern "C" int oec_furman_emit(const oec_furman_t *params, const double *rows_de
         return OEC_ERR_INVALID;
     if (cap > kMaxAbsorbedRows) return OEC_ERR_INVALID;
     cudaStream_t s = as_stream(stream);
-    // work layout: Rec[cap] | split[cap * kSlots] (f64) | nsec[cap] | offset[cap] | partial[scan_blocks(cap)]
+    // work layout: SplitConst | Rec[cap] | split[cap * kSlots] (f64) | nsec[cap] | offset[cap] |
+    // partial[scan_blocks(cap)]
     char *w = static_cast<char *>(work_dev);
-    Rec *rec = reinterpret_cast<Rec *>(w);
-    double *split = reinterpret_cast<double *>(w + sizeof(Rec) * (size_t)cap);
+    SplitConst *consts = reinterpret_cast<SplitConst *>(w);
+    Rec *rec = reinterpret_cast<Rec *>(w + sizeof(SplitConst));
+    double *split = reinterpret_cast<double *>(rec + cap);
     int32_t *nsec = reinterpret_cast<int32_t *>(split + (size_t)cap * kSlots);
     int32_t *off = nsec + cap;
     int *partial = off + cap;
     uint2 key = make_uint2((uint32_t)seed, (uint32_t)(seed >> 32));
-    int g = persistent_grid((cap + 127) / 128, 8);
-    k_furman_pass1<<<g, 128, 0, s>>>(*params, rows_dev, normals_dev, n_abs_dev, cap, ids_dev, key, step, step_dev,
-                                     replay_uniforms_dev, rec, nsec, status_dev);
+    const int g = persistent_grid((cap + 127) / 128, 8);
+    k_furman_pass1<<<g + kClasses + kSlots, 128, 0, s>>>(*params, rows_dev, normals_dev, n_abs_dev, cap, ids_dev, key, step,
+                                                step_dev, replay_uniforms_dev, rec, nsec, status_dev, g, consts);
     if (cap > 0) {
         scan_counts(nsec, n_abs_dev, cap, off, partial, n_out_dev, s);
     } else {
         OEC_CUDA_TRY(cudaMemsetAsync(n_out_dev, 0, sizeof(int32_t), s));
     }
-    k_furman_pass2a<<<persistent_grid(((int64_t)cap * kSlots + 127) / 128, 8), 128, 0, s>>>(
-        *params, n_abs_dev, cap, ids_dev, key, step, step_dev, replay_uniforms_dev, rec, split);
-    k_furman_pass2<<<g, 128, 0, s>>>(*params, rows_dev, normals_dev, n_abs_dev, cap, ids_dev, key, step, step_dev,
-                                     replay_uniforms_dev, rec, split, off, out_rows_dev, out_cap, status_dev);
+    static std::atomic<int> attr[kMaxDevices];
+    const int ok = per_device_cached(attr, [] {
+        return cudaFuncSetAttribute(k_furman_emit, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)sizeof(SplitShared)) == cudaSuccess
+                   ? 1
+                   : 0;
+    });
+    if (!ok) return OEC_ERR_CUDA;
+    k_furman_emit<<<persistent_grid((cap + 31) / 32, 2), kSplitT, sizeof(SplitShared), s>>>(
+        *params, rows_dev, normals_dev, n_abs_dev, cap, ids_dev, key, step, step_dev, replay_uniforms_dev, rec,
+        consts, split, off, out_rows_dev, out_cap, status_dev);
     OEC_LAUNCH_CHECK();
     return OEC_OK;
 }
@@ -615,7 +717,7 @@ extern "C" int64_t oec_secelec_work_bytes(int32_t cap) {
 
 extern "C" int64_t oec_furman_work_bytes(int32_t cap) {
     if (cap < 0 || cap > kMaxAbsorbedRows) return -1;
-    return (int64_t)sizeof(Rec) * cap + (int64_t)sizeof(double) * kSlots * cap + 2 * sizeof(int32_t) * (int64_t)cap +
+    return (int64_t)sizeof(SplitConst) + (int64_t)sizeof(Rec) * cap + (int64_t)sizeof(double) * kSlots * cap + 2 * sizeof(int32_t) * (int64_t)cap +
            sizeof(int) * (int64_t)scan_blocks(cap) + 256;
 }
 
