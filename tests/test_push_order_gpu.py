@@ -1,0 +1,47 @@
+"""The fused step on stores in cell order and in random order.
+
+A CTA decides from its first chunk whether its particles are near each other
+(windows in shared memory) or not (pairs of lanes straight to the grid).  Both
+give the same particles and the same integer deposit, so a random order and
+the cell order of the same rows must agree bit for bit."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _step(rows, bound, btype):
+    import torch
+    from openecloud_b200.grid import Grid
+    from openecloud_b200.particleBoundary import AbsorbElliptical, AbsorbRectangular
+    from openecloud_b200.particles import Particles
+    g = Grid(150, 220, 0.04, 0.06, bound)
+    P = Particles("electrons", "variableWeight")
+    P.setBConst([0.0, 0.5, 0.0])
+    P.setParticleData(rows)
+    P._bind(g)
+    G = g.getNpExt()
+    e = P.fieldTable(g, np.random.default_rng(1).normal(0, 1e4, 2 * G), 2)
+    b = P.fieldTable(g, np.random.default_rng(2).normal(0, 0.1, 3 * G), 3) if btype == 2 else None
+    bd = (AbsorbRectangular if bound == 0 else AbsorbElliptical)(g, P)
+    P.pushGatherDeposit(g, e, 3e-11, btype, bd, bCellTable=b)
+    torch.cuda.synchronize()
+    fix, scale = P.getChargeOnGridFixed()
+    return P.getParticleData(), P.getIsInside(), fix, scale
+
+
+@pytest.mark.parametrize("bound,btype", [(0, 0), (1, 1), (1, 2)])
+@pytest.mark.parametrize("n", [1, 2, 33, 1023, 1024, 1025, 2047, 50_001])
+def test_random_and_cell_order_agree(gpu, n, bound, btype):
+    rng = np.random.default_rng(n)
+    rows = np.empty((n, 6))
+    rows[:, 0], rows[:, 1] = rng.uniform(-0.0199, 0.0199, n), rng.uniform(-0.0299, 0.0299, n)
+    rows[:, 2:5] = rng.normal(0, 2e6, (n, 3))
+    rows[:, 5] = rng.uniform(0.5, 2.0, n)
+    order = np.lexsort((rows[:, 0], np.floor(rows[:, 1] / (0.06 / 219))))
+    a, ina, fa, sa = _step(rows, bound, btype)
+    b, inb, fb, sb = _step(rows[order], bound, btype)
+    assert sa == sb and np.array_equal(fa, fb)
+    assert np.array_equal(a[order], b) and np.array_equal(ina[order], inb)
+    # the deposit is exact: every survivor's whole quantised charge is on the grid
+    assert fa.sum() == np.rint(rows[ina == 1, 5].astype(np.float32).astype(np.float64) * sa).sum()
