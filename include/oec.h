@@ -427,25 +427,29 @@ int oec_cell_merge(const oec_grid_t *grid, oec_particles_t *p, int32_t n_cand, i
 /* Nested-dissection fronts of A (nd_setup.py): the form in which the direct
  * solve normally runs.  A front has s pivots and b boundary unknowns (pivots of
  * fronts above it); its blocks are X = A11^-1 and G = A21 X, stored input by
- * input: [X | G^T] as s rows of ldf values from mat + mf, G as b rows of ldb
- * values from mat + mb (ldf, ldb, mf, mb even).  Level 0 is the one front at the
- * root; forward runs from level n_levels - 1 to 0, backward from 1 on.  A tile
- * is (front, first output); width 8, 16, 32 or 64 outputs are a CTA's work, width
- * 0 gives a whole front (at most 256 inputs) to a warp.  piv_src / bnd_src hold,
- * per pivot / boundary entry, up to four entries of u that its children left
- * for it (-1: none).  Pointers are device pointers (host ones in
- * oec_lu_host_t). */
+ * input: forward [X | G^T] as s rows of ld values, backward G as b rows of ld
+ * values (ld and every block's place even).  Level 0 is the one front at the
+ * root; forward runs from level n_levels - 1 to 0, backward from 1 on.  A tile is
+ * n_out outputs from o0 on of one front in one direction.  The tiles of a pass are
+ * taken by groups of 512 threads (n_out <= width <= 256, n_in <= max_front), of 128
+ * (n_out <= width <= 128, n_in <= max_front / 4), or by warps (whole fronts, n_in <=
+ * OEC_ND_WARP_IN); width is a power of two from 8 on.  piv_src / bnd_src hold, per
+ * pivot / boundary entry, up to four entries of u that its children left for it
+ * (-1: none).  Pointers are device pointers (host ones in oec_lu_host_t). */
 #define OEC_ND_MAX_LEVELS 16
 #define OEC_ND_MAX_FRONT 6144
-typedef struct oec_nd_front {
-    int32_t s, b;
-    int32_t piv0, bnd0;        /* first entry in piv_node / bnd_node (and y / u) */
-    int32_t ldf, ldb;
-    int64_t mf, mb;
-} oec_nd_front_t;
+#define OEC_ND_WARP_IN 32
+typedef struct oec_nd_tile {
+    int64_t mat;               /* input 0, output o0 in mat */
+    int32_t n_in, n_out, ld, o0;
+    int32_t piv0, bnd0;        /* the front's first entry in piv_node (and y) / bnd_node (and u) */
+} oec_nd_tile_t;
+typedef struct oec_nd_pass {
+    int32_t tile, tiles;       /* first tile, tiles */
+    int32_t width, group;      /* outputs per tile; threads per group: 512, 128 or 32 */
+} oec_nd_pass_t;
 typedef struct oec_nd_level {
-    int32_t fwd_tile, fwd_tiles, fwd_width;
-    int32_t bwd_tile, bwd_tiles, bwd_width;
+    oec_nd_pass_t fwd, bwd;
     int32_t has_children;      /* some front of the level has fronts below it */
     int32_t pad;
 } oec_nd_level_t;
@@ -455,19 +459,18 @@ typedef struct oec_nd {
     int32_t n_bnd;             /* boundary entries of all fronts */
     int32_t n_outside;         /* nodes that are no unknown (phi = 0) */
     int32_t n_levels;
-    int32_t max_front;         /* largest s or b */
-    int32_t n_fronts;
+    int32_t max_front;         /* inputs that a CTA's shared memory holds: at least 16 * OEC_ND_WARP_IN, a multiple of 4 */
     int32_t n_tiles;
+    int32_t pad;
     int64_t n_mat;
     oec_nd_level_t level[OEC_ND_MAX_LEVELS];
-    const oec_nd_front_t *fronts; /* [n_fronts] */
-    const int32_t *tiles;      /* [2 * n_tiles] */
+    const oec_nd_tile_t *tiles; /* [n_tiles], 16-byte aligned */
     const int32_t *piv_node;   /* [n] */
-    const int32_t *piv_src;    /* [4 * n] */
+    const int32_t *piv_src;    /* [4 * n], 16-byte aligned */
     const int32_t *bnd_node;   /* [n_bnd] */
-    const int32_t *bnd_src;    /* [4 * n_bnd] */
+    const int32_t *bnd_src;    /* [4 * n_bnd], 16-byte aligned */
     const int32_t *outside;    /* [n_outside] */
-    const double *mat;         /* [n_mat] */
+    const double *mat;         /* [n_mat], 16-byte aligned */
 } oec_nd_t;
 
 /* Device form of SuperLU's P_r A P_c = L U (poissonSolver.pyx:59).

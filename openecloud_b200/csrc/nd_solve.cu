@@ -14,9 +14,12 @@
 // block times a vector.  The bytes of the blocks bound large grids, the
 // barriers and the dependent loads around them small ones.  Measured (warm,
 // per solve) against the level-scheduled factors with their dense tail:
-// 33 x 25 rectangle 11.5 against 270 us, 128^2 circle 31 against 146 us, 512^2
-// ellipse 168 against 1400 us, 1024^2 ellipse 451 us against 9.1 ms; the blocks
-// take 4, 44, 318 and 1144 MB (the 1024^2 tail inverses alone took 4.3 GB).
+// 33 x 25 rectangle 6.2 against 270 us, 128^2 circle 20.5 against 146 us, 512^2
+// ellipse 115 against 1400 us, 1024^2 ellipse 320 us against 9.1 ms; the blocks
+// take 4, 44, 264 and 1049 MB (the 1024^2 tail inverses alone took 4.3 GB).
+// Tried and dropped: only 128-thread CTAs, eight to an SM (45 us at 128^2: every
+// CTA gathers a long front's inputs anew); fetching the next pass's first blocks
+// into L1 or L2 ahead of the barrier (1024^2 330 -> 344 us).
 #include <stdint.h>
 
 #include <cooperative_groups.h>
@@ -30,8 +33,8 @@ namespace {
 
 constexpr int kNdThreads = 512, kNdWarps = kNdThreads / 32;
 constexpr int kNdPerSm = 2;       // resident CTAs per SM
-constexpr int kNdWarpVec = 256;   // inputs of a front that one warp takes
-constexpr int kNdWidth = 64;      // widest tile of a CTA
+constexpr int kNdQuarter = 128;   // threads of a group that is a quarter of a CTA
+constexpr int kNdWarpVec = OEC_ND_WARP_IN;
 
 struct NdArgs {
     oec_nd_t nd;
@@ -41,177 +44,247 @@ struct NdArgs {
 
 __device__ __forceinline__ double2 load_mat(const double *p) { return __ldg(reinterpret_cast<const double2 *>(p)); }
 
+__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
+__device__ __forceinline__ oec_nd_tile_t load_tile(const oec_nd_tile_t *p) {
+    union {
+        int4 v[2];
+        oec_nd_tile_t t;
+    } x;
+    x.v[0] = __ldg(reinterpret_cast<const int4 *>(p));
+    x.v[1] = __ldg(reinterpret_cast<const int4 *>(p) + 1);
+    return x.t;
+}
+
 // Sum of the (at most four) child updates that go to one entry.  The order is
 // the setup's, so the sum does not depend on the launch.
-__device__ __forceinline__ double child_sum(const int4 *__restrict__ src, int e, const double *u) {
-    const int4 k = __ldg(src + e);
-    double a = 0.0;
-    if (k.x >= 0) a = __ldcg(u + k.x);
-    if (k.y >= 0) a += __ldcg(u + k.y);
-    if (k.z >= 0) a += __ldcg(u + k.z);
-    if (k.w >= 0) a += __ldcg(u + k.w);
-    return a;
+__device__ __forceinline__ double child_sum(const int4 k, const double *u) {
+    const double a = k.x >= 0 ? __ldcg(u + k.x) : 0.0, b = k.y >= 0 ? __ldcg(u + k.y) : 0.0;
+    const double c = k.z >= 0 ? __ldcg(u + k.z) : 0.0, d = k.w >= 0 ? __ldcg(u + k.w) : 0.0;
+    return ((a + b) + c) + d;
 }
 
-// Partial products of 2 outputs at o with the inputs i0, i0 + step, ... < n.
-// The block is stored input by input, so the lanes of a warp read neighbouring
-// outputs of one input and no product needs a reduction inside a row.
-__device__ __forceinline__ double2 partial(const double *__restrict__ M, int ld, int o, int i0, int step, int n,
+// Partial products of 2 outputs with the inputs i0, i0 + step, ... < n; M at the
+// outputs' place in input 0.  The block is stored input by input, so the lanes of
+// a warp read neighbouring outputs of one input and no product needs a
+// reduction inside a row.
+template <int U>  // loads in flight per lane
+__device__ __forceinline__ double2 partial(const double *__restrict__ M, int ld, int i0, int step, int n,
                                            const double *vec) {
     double2 a = make_double2(0.0, 0.0);
-    const double *p = M + (int64_t)i0 * ld + o;
+    const double *p = M + (int64_t)i0 * ld;
     const int64_t d = (int64_t)step * ld;
     int i = i0;
-    for (; i + 3 * step < n; i += 4 * step, p += 4 * d) {
-        const double2 m0 = load_mat(p), m1 = load_mat(p + d), m2 = load_mat(p + 2 * d), m3 = load_mat(p + 3 * d);
-        const double v0 = vec[i], v1 = vec[i + step], v2 = vec[i + 2 * step], v3 = vec[i + 3 * step];
-        a.x += m0.x * v0;
-        a.y += m0.y * v0;
-        a.x += m1.x * v1;
-        a.y += m1.y * v1;
-        a.x += m2.x * v2;
-        a.y += m2.y * v2;
-        a.x += m3.x * v3;
-        a.y += m3.y * v3;
+    for (; i + (U - 1) * step < n; i += U * step, p += U * d) {
+        double2 m[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) m[k] = load_mat(p + k * d);
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const double v = vec[i + k * step];
+            a.x += m[k].x * v;
+            a.y += m[k].y * v;
+        }
     }
-    for (; i < n; i += step, p += d) {
-        const double2 m = load_mat(p);
-        const double v = vec[i];
-        a.x += m.x * v;
-        a.y += m.y * v;
-    }
+    // the last ones, loaded together
+    double2 m[U - 1];
+#pragma unroll
+    for (int k = 0; k < U - 1; ++k) m[k] = i + k * step < n ? load_mat(p + k * d) : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int k = 0; k < U - 1; ++k)
+        if (i + k * step < n) {
+            const double v = vec[i + k * step];
+            a.x += m[k].x * v;
+            a.y += m[k].y * v;
+        }
     return a;
 }
 
+// The inputs of a tile into v: forward the pivots' right-hand side with the
+// children's updates, backward phi on the boundary.
 template <bool FWD>
-__device__ __forceinline__ double gather_in(const NdArgs &a, const oec_nd_front_t &f, int i, bool children) {
-    if (FWD) {
-        double v = __ldg(a.q + __ldg(a.nd.piv_node + f.piv0 + i));
-        if (children) v += child_sum(reinterpret_cast<const int4 *>(a.nd.piv_src), f.piv0 + i, a.u);
-        return v;
-    }
-    return __ldcg(a.phi + __ldg(a.nd.bnd_node + f.bnd0 + i));
-}
-
-template <bool FWD>
-__device__ __forceinline__ void put_out(const NdArgs &a, const oec_nd_front_t &f, int o, double val, bool children,
-                                        bool root) {
-    if (FWD) {
-        if (o < f.s) {
-            if (root)
-                a.phi[__ldg(a.nd.piv_node + f.piv0 + o)] = val;
-            else
-                a.y[f.piv0 + o] = val;
-        } else if (o < f.s + f.b) {
-            const int e = f.bnd0 + o - f.s;
-            const double v = children ? child_sum(reinterpret_cast<const int4 *>(a.nd.bnd_src), e, a.u) : 0.0;
-            a.u[e] = v - val;
+__device__ __forceinline__ void gather(const NdArgs &a, const oec_nd_tile_t &t, bool children, int first, int step,
+                                       double *v) {
+    const int4 *src = reinterpret_cast<const int4 *>(a.nd.piv_src) + t.piv0;
+    const int32_t *node = FWD ? a.nd.piv_node + t.piv0 : a.nd.bnd_node + t.bnd0;
+#pragma unroll 2
+    for (int i = first; i < t.n_in; i += step) {
+        const int k = __ldg(node + i);
+        if (FWD) {
+            double x = __ldg(a.q + k);
+            if (children) x += child_sum(__ldg(src + i), a.u);
+            v[i] = x;
+        } else {
+            v[i] = __ldcg(a.phi + k);
         }
-    } else if (o < f.s) {
-        a.phi[__ldg(a.nd.piv_node + f.piv0 + o)] = __ldcg(a.y + f.piv0 + o) - val;
     }
 }
 
-// One direction of one level.  width > 0: a tile is `width` outputs of a front,
-// its inputs split over the 16 warps of a CTA (summed in a fixed order);
-// width 0: a tile is a whole front, one warp's work.
+// What a product at output o is combined with, read before the product is
+// there: y of the backward direction, the children's updates to a boundary entry
+// of the forward one.
 template <bool FWD>
-__device__ __forceinline__ void run_level(const NdArgs &a, const int2 *__restrict__ tiles, int n_tiles, int width,
-                                          bool children, bool root, double *vec, double *red) {
+__device__ __forceinline__ double out_base(const NdArgs &a, const oec_nd_tile_t &t, int o, bool children) {
+    if (o >= t.o0 + t.n_out) return 0.0;
+    if (!FWD) return __ldcg(a.y + t.piv0 + o);
+    if (!children || o < t.n_in) return 0.0;
+    return child_sum(__ldg(reinterpret_cast<const int4 *>(a.nd.bnd_src) + t.bnd0 + o - t.n_in), a.u);
+}
+
+template <bool FWD>
+__device__ __forceinline__ void put_out(const NdArgs &a, const oec_nd_tile_t &t, int o, double base, double val,
+                                        bool root) {
+    if (o >= t.o0 + t.n_out) return;
+    if (!FWD)
+        a.phi[__ldg(a.nd.piv_node + t.piv0 + o)] = base - val;
+    else if (o >= t.n_in)
+        a.u[t.bnd0 + o - t.n_in] = base - val;
+    else if (root)
+        a.phi[__ldg(a.nd.piv_node + t.piv0 + o)] = val;
+    else
+        a.y[t.piv0 + o] = val;
+}
+
+// A barrier of a group of GT threads: the CTA's, or one of its quarters'.
+template <int GT>
+__device__ __forceinline__ void group_sync() {
+    if (GT == kNdThreads)
+        __syncthreads();
+    else
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / GT), "n"(GT) : "memory");
+}
+
+// The tiles of one direction of one level by groups of GT threads.  A tile is
+// `width` outputs of a front; its inputs are split over the lanes that the
+// outputs leave (summed in a fixed order).  What a tile costs is its chain of
+// dependent loads (tile, indices, values, block): quarter CTAs have four times
+// as many chains under way, whole ones gather long inputs faster.
+template <bool FWD, int GT>
+__device__ __forceinline__ void run_tiles(const NdArgs &a, const oec_nd_tile_t *__restrict__ tiles, int n_tiles,
+                                          int width, bool children, bool root, double *vec, double *red) {
+    constexpr int kGroups = kNdThreads / GT, kWarps = GT / 32;
+    const int lane = threadIdx.x & 31, group = threadIdx.x / GT, tid = threadIdx.x % GT;
+    const int L = width >> 1, parts = GT / L;  // L lanes across the outputs, two each
+    const int part = tid / L, col = tid & (L - 1);
+    const int slots = L < 32 ? kWarps : parts, slot = L < 32 ? tid >> 5 : part;
+    vec += group * (a.nd.max_front / kGroups);
+    red += group * 2 * GT;
+    const int step = gridDim.x * kGroups;
+    for (int k = blockIdx.x + group * gridDim.x; k < n_tiles; k += step) {
+        const oec_nd_tile_t t = load_tile(tiles + k);
+        if (tid == 0 && k + step < n_tiles) prefetch_l1(tiles + k + step);
+        gather<FWD>(a, t, children, tid, GT, vec);
+        const int oa = t.o0 + tid;  // this thread's output
+        const bool has = tid < width;
+        const double base = has ? out_base<FWD>(a, t, oa, children) : 0.0;
+        group_sync<GT>();
+        double2 s = make_double2(0.0, 0.0);
+        if (t.o0 + 2 * col < t.ld) s = partial<4>(a.nd.mat + t.mat + 2 * col, t.ld, part, parts, t.n_in, vec);
+        for (int m = 16; m >= L; m >>= 1) {
+            s.x += __shfl_xor_sync(kFullMask, s.x, m);
+            s.y += __shfl_xor_sync(kFullMask, s.y, m);
+        }
+        if (L >= 32 || lane < L) *reinterpret_cast<double2 *>(red + slot * width + 2 * col) = s;
+        group_sync<GT>();
+        if (has) {
+            double v = 0.0;
+            for (int m = 0; m < slots; ++m) v += red[m * width + tid];
+            put_out<FWD>(a, t, oa, base, v, root);
+        }
+        // red is written again only behind the next tile's first barrier, vec behind this one's last read
+    }
+}
+
+// The tiles by single warps: whole fronts of at most kNdWarpVec inputs.
+template <bool FWD>
+__device__ __forceinline__ void run_fronts(const NdArgs &a, const oec_nd_tile_t *__restrict__ tiles, int n_tiles,
+                                           bool children, bool root, double *vec) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (width == 0) {
-        double *v = vec + warp * kNdWarpVec;
-        for (int t = blockIdx.x * kNdWarps + warp; t < n_tiles; t += gridDim.x * kNdWarps) {
-            const oec_nd_front_t f = a.nd.fronts[__ldg(&tiles[t].x)];
-            const int n_in = FWD ? f.s : f.b, n_out = FWD ? f.s + f.b : f.s, ld = FWD ? f.ldf : f.ldb;
-            const double *M = a.nd.mat + (FWD ? f.mf : f.mb);
-            __syncwarp();
-            for (int i = lane; i < n_in; i += 32) v[i] = gather_in<FWD>(a, f, i, children);
-            __syncwarp();
-            const int L = n_out > 32 ? 32 : n_out > 16 ? 16 : 8;  // lanes across the outputs, two each
-            const int R = 32 / L, sub = lane / L, ol = 2 * (lane & (L - 1));
-            for (int o0 = 0; o0 < n_out; o0 += 2 * L) {
-                const int o = o0 + ol;
-                double2 s = make_double2(0.0, 0.0);
-                if (o < ld) s = partial(M, ld, o, sub, R, n_in, v);
-                for (int k = 16; k >= L; k >>= 1) {
-                    s.x += __shfl_xor_sync(kFullMask, s.x, k);
-                    s.y += __shfl_xor_sync(kFullMask, s.y, k);
-                }
-                if (sub == 0) {
-                    put_out<FWD>(a, f, o, s.x, children, root);
-                    put_out<FWD>(a, f, o + 1, s.y, children, root);
-                }
+    double *v = vec + warp * kNdWarpVec;
+    const int step = gridDim.x * kNdWarps;
+    for (int k = blockIdx.x * kNdWarps + warp; k < n_tiles; k += step) {
+        const oec_nd_tile_t t = load_tile(tiles + k);
+        if (k + step < n_tiles) prefetch_l1(tiles + k + step);
+        __syncwarp();
+        gather<FWD>(a, t, children, lane, 32, v);
+        __syncwarp();
+        const int L = t.n_out > 32 ? 32 : t.n_out > 16 ? 16 : 8;  // lanes across the outputs, two each
+        const int R = 32 / L, sub = lane / L, ol = 2 * (lane & (L - 1));
+        for (int o0 = 0; o0 < t.n_out; o0 += 2 * L) {
+            const int o = o0 + ol;
+            const double b0 = sub == 0 ? out_base<FWD>(a, t, o, children) : 0.0;
+            const double b1 = sub == 0 ? out_base<FWD>(a, t, o + 1, children) : 0.0;
+            double2 s = make_double2(0.0, 0.0);
+            if (o < t.ld) s = partial<6>(a.nd.mat + t.mat + o, t.ld, sub, R, t.n_in, v);
+            for (int m = 16; m >= L; m >>= 1) {
+                s.x += __shfl_xor_sync(kFullMask, s.x, m);
+                s.y += __shfl_xor_sync(kFullMask, s.y, m);
+            }
+            if (sub == 0) {
+                put_out<FWD>(a, t, o, b0, s.x, root);
+                put_out<FWD>(a, t, o + 1, b1, s.y, root);
             }
         }
-        return;
     }
-    const int L = width >> 1, R = 32 / L, sub = lane / L, ol = 2 * (lane & (L - 1));
-    for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-        const int2 tile = __ldg(tiles + t);
-        const oec_nd_front_t f = a.nd.fronts[tile.x];
-        const int n_in = FWD ? f.s : f.b, ld = FWD ? f.ldf : f.ldb;
-        const double *M = a.nd.mat + (FWD ? f.mf : f.mb);
-        for (int i = threadIdx.x; i < n_in; i += kNdThreads) vec[i] = gather_in<FWD>(a, f, i, children);
-        __syncthreads();
-        const int o = tile.y + ol;
-        double2 s = make_double2(0.0, 0.0);
-        if (o < ld) s = partial(M, ld, o, warp * R + sub, kNdWarps * R, n_in, vec);
-        for (int k = 16; k >= L; k >>= 1) {
-            s.x += __shfl_xor_sync(kFullMask, s.x, k);
-            s.y += __shfl_xor_sync(kFullMask, s.y, k);
-        }
-        if (sub == 0) *reinterpret_cast<double2 *>(red + warp * kNdWidth + ol) = s;
-        __syncthreads();
-        if (threadIdx.x < width) {
-            double v = 0.0;
-#pragma unroll
-            for (int k = 0; k < kNdWarps; ++k) v += red[k * kNdWidth + threadIdx.x];
-            put_out<FWD>(a, f, tile.y + threadIdx.x, v, children, root);
-        }
-        __syncthreads();
-    }
+}
+
+template <bool FWD>
+__device__ __forceinline__ void run_level(const NdArgs &a, const oec_nd_pass_t &p, bool children, bool root,
+                                          double *vec, double *red) {
+    if (p.group == kNdThreads)
+        run_tiles<FWD, kNdThreads>(a, a.nd.tiles + p.tile, p.tiles, p.width, children, root, vec, red);
+    else if (p.group == kNdQuarter)
+        run_tiles<FWD, kNdQuarter>(a, a.nd.tiles + p.tile, p.tiles, p.width, children, root, vec, red);
+    else
+        run_fronts<FWD>(a, a.nd.tiles + p.tile, p.tiles, children, root, vec);
 }
 
 __global__ void __launch_bounds__(kNdThreads, kNdPerSm) k_nd_solve(const __grid_constant__ NdArgs a) {
-    extern __shared__ double vec[];
-    __shared__ __align__(16) double red[kNdWarps * kNdWidth];
+    extern __shared__ __align__(16) double vec[];
+    __shared__ __align__(16) double red[2 * kNdThreads];  // (split of the inputs) x width
     cooperative_groups::grid_group grid = cooperative_groups::this_grid();
-    const int2 *tiles = reinterpret_cast<const int2 *>(a.nd.tiles);
     for (int i = blockIdx.x * kNdThreads + threadIdx.x; i < a.nd.n_outside; i += gridDim.x * kNdThreads)
         a.phi[a.nd.outside[i]] = 0.0;
     for (int k = a.nd.n_levels - 1; k >= 0; --k) {
         const oec_nd_level_t &l = a.nd.level[k];
-        run_level<true>(a, tiles + l.fwd_tile, l.fwd_tiles, l.fwd_width, l.has_children != 0, k == 0, vec, red);
+        run_level<true>(a, l.fwd, l.has_children != 0, k == 0, vec, red);
         if (a.nd.n_levels > 1) grid.sync();
     }
     for (int k = 1; k < a.nd.n_levels; ++k) {
-        const oec_nd_level_t &l = a.nd.level[k];
-        run_level<false>(a, tiles + l.bwd_tile, l.bwd_tiles, l.bwd_width, false, false, vec, red);
+        run_level<false>(a, a.nd.level[k].bwd, false, false, vec, red);
         if (k + 1 < a.nd.n_levels) grid.sync();
     }
 }
 
-bool width_ok(int w) { return w == 0 || w == 8 || w == 16 || w == 32 || w == 64; }
+// A pass fits the kernel: its tiles exist, its group is one of the three and its
+// width a power of two that the group's lanes can take.
+bool pass_ok(const oec_nd_pass_t &p, int n_tiles) {
+    if (p.tile < 0 || p.tiles < 0 || (int64_t)p.tile + p.tiles > n_tiles) return false;
+    if (p.group == 32) return true;
+    return (p.group == kNdThreads || p.group == kNdQuarter) && p.width >= 8 && (p.width & (p.width - 1)) == 0 &&
+           p.width <= (p.group == kNdThreads ? 256 : 128);
+}
+
+int64_t pass_ctas(const oec_nd_pass_t &p) {
+    const int groups = kNdThreads / p.group;
+    return (p.tiles + groups - 1) / groups;
+}
 
 }  // namespace
 
 int nd_solve(const oec_nd_t *nd, const double *q, double *phi, double *work, cudaStream_t s) {
-    if (nd->n <= 0 || nd->n_levels < 1 || nd->n_levels > OEC_ND_MAX_LEVELS || nd->max_front < 1 ||
-        nd->max_front > OEC_ND_MAX_FRONT || nd->n_bnd < 0 || nd->n_outside < 0 || !nd->fronts || !nd->tiles ||
-        !nd->piv_node || !nd->mat || (nd->n_levels > 1 && (!nd->piv_src || !nd->bnd_node || !nd->bnd_src)) ||
+    if (nd->n <= 0 || nd->n_levels < 1 || nd->n_levels > OEC_ND_MAX_LEVELS || nd->max_front < kNdWarps * kNdWarpVec ||
+        nd->max_front > OEC_ND_MAX_FRONT || nd->max_front % 4 || nd->n_bnd < 0 || nd->n_outside < 0 || !nd->tiles || !nd->piv_node ||
+        !nd->mat || (nd->n_levels > 1 && (!nd->piv_src || !nd->bnd_node || !nd->bnd_src)) ||
         (nd->n_outside > 0 && !nd->outside))
         return OEC_ERR_INVALID;
     int64_t need = 1;
     for (int k = 0; k < nd->n_levels; ++k) {
         const oec_nd_level_t &l = nd->level[k];
-        if (!width_ok(l.fwd_width) || !width_ok(l.bwd_width) || l.fwd_tile < 0 || l.bwd_tile < 0 ||
-            l.fwd_tile + (int64_t)l.fwd_tiles > nd->n_tiles || l.bwd_tile + (int64_t)l.bwd_tiles > nd->n_tiles)
-            return OEC_ERR_INVALID;
-        need = std::max<int64_t>(need, l.fwd_width ? l.fwd_tiles : (l.fwd_tiles + kNdWarps - 1) / kNdWarps);
-        need = std::max<int64_t>(need, l.bwd_width ? l.bwd_tiles : (l.bwd_tiles + kNdWarps - 1) / kNdWarps);
+        if (!pass_ok(l.fwd, nd->n_tiles) || !pass_ok(l.bwd, nd->n_tiles)) return OEC_ERR_INVALID;
+        need = std::max(need, std::max(pass_ctas(l.fwd), pass_ctas(l.bwd)));
     }
-    const size_t smem = sizeof(double) * (size_t)std::max(nd->max_front, kNdWarps * kNdWarpVec);
+    const size_t smem = sizeof(double) * (size_t)nd->max_front;
     static std::atomic<int> attr[kMaxDevices];
     const int ok = per_device_cached(attr, [] {
         return cudaFuncSetAttribute(k_nd_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -221,14 +294,18 @@ int nd_solve(const oec_nd_t *nd, const double *q, double *phi, double *work, cud
     });
     if (!ok) return OEC_ERR_CUDA;
     NdArgs a{*nd, q, phi, work, work + nd->n};
-    const int grid = (int)std::min<int64_t>(need, (int64_t)sm_count() * kNdPerSm);
-    if (nd->n_levels == 1) {
-        k_nd_solve<<<grid, kNdThreads, smem, s>>>(a);
+    if (nd->n_levels == 1) {  // no barrier: an ordinary launch
+        k_nd_solve<<<(unsigned)need, kNdThreads, smem, s>>>(a);
         OEC_LAUNCH_CHECK();
-    } else {
-        void *args[] = {&a};
-        OEC_CUDA_TRY(cudaLaunchCooperativeKernel((void *)k_nd_solve, dim3(grid), dim3(kNdThreads), args, smem, s));
+        return OEC_OK;
     }
+    // every CTA resident at once: the barrier between levels is the grid's
+    int per_sm = 0;
+    OEC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_nd_solve, kNdThreads, smem));
+    const int grid = (int)std::min<int64_t>(need, (int64_t)sm_count() * std::min(per_sm, kNdPerSm));
+    if (grid < 1) return OEC_ERR_CUDA;
+    void *args[] = {&a};
+    OEC_CUDA_TRY(cudaLaunchCooperativeKernel((void *)k_nd_solve, dim3(grid), dim3(kNdThreads), args, smem, s));
     return OEC_OK;
 }
 

@@ -219,7 +219,7 @@ bool valid_desc(const oec_run_desc_t *d) {
            (d->boundary_kind == OEC_BOUNDARY_RECT || d->boundary_kind == OEC_BOUNDARY_ELLIPSE) &&
            (d->type_b == 0 || d->type_b == 1) && d->mass > 0 && L.n >= 1 && L.head >= 0 && L.head <= L.n &&
            L.n_nodes == d->grid.nx * d->grid.ny && d->e_ptr && d->e_idx && d->e_val &&
-           (L.nd ? L.nd->n == L.n && L.nd->n_nodes == L.n_nodes && L.nd->n_fronts >= 1 && L.nd->n_tiles >= 1 &&
+           (L.nd ? L.nd->n == L.n && L.nd->n_nodes == L.n_nodes && L.nd->n_tiles >= 1 &&
                        L.nd->n_bnd >= 0 && L.nd->n_outside >= 0 && L.nd->n_mat >= 1
                  : L.l_level_ptr && L.u_level_ptr && L.rhs_node && L.sol_src && L.sol_node);
 }
@@ -264,9 +264,8 @@ int create_run(oec_ctx *c, const oec_run_desc_t *d, oec_run *r) {
     if (L.nd) {
         r->nd = *L.nd;
         const oec_nd_t &h = *L.nd;
-        oec_nd_front_t *fr;
-        OEC_TRY(ctx_upload(c, h.fronts, h.n_fronts, &fr)); r->nd.fronts = fr;
-        OEC_TRY(ctx_upload(c, h.tiles, 2 * (size_t)h.n_tiles, &i32)); r->nd.tiles = i32;
+        oec_nd_tile_t *tiles;
+        OEC_TRY(ctx_upload(c, h.tiles, h.n_tiles, &tiles)); r->nd.tiles = tiles;
         OEC_TRY(ctx_upload(c, h.piv_node, h.n, &i32)); r->nd.piv_node = i32;
         OEC_TRY(ctx_upload(c, h.piv_src, 4 * (size_t)h.n, &i32)); r->nd.piv_src = i32;
         OEC_TRY(ctx_upload(c, h.bnd_node, h.n_bnd, &i32)); r->nd.bnd_node = i32;

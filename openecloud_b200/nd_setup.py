@@ -24,26 +24,30 @@ from . import _lib
 
 MAX_LEVELS = 16       # oec_nd_t's array of levels
 MAX_FRONT = 6144      # pivots or boundary unknowns of one front (the device keeps them in shared memory)
-WARP_FRONT = 256      # fronts of at most this many inputs may be taken by one warp each
+WARP_IN = 32          # fronts of at most this many inputs may be taken by one warp each
+QUARTER_IN = 512      # and of this many by a quarter of a CTA
+CTAS = 296            # CTAs of 512 threads that solve together: 2 on each of a B200's 148 SMs
 LEAF = 12             # unknowns below which a set is not split
 
 
+class NdPass_t(ctypes.Structure):
+    _fields_ = [(k, ctypes.c_int32) for k in ("tile", "tiles", "width", "group")]
+
+
 class NdLevel_t(ctypes.Structure):
-    _fields_ = [(k, ctypes.c_int32) for k in ("fwd_tile", "fwd_tiles", "fwd_width", "bwd_tile", "bwd_tiles",
-                                              "bwd_width", "has_children", "pad")]
+    _fields_ = [("fwd", NdPass_t), ("bwd", NdPass_t), ("has_children", ctypes.c_int32), ("pad", ctypes.c_int32)]
 
 
 class Nd_t(ctypes.Structure):
     _P = ctypes.c_void_p
     _fields_ = [("n", ctypes.c_int32), ("n_nodes", ctypes.c_int32), ("n_bnd", ctypes.c_int32),
                 ("n_outside", ctypes.c_int32), ("n_levels", ctypes.c_int32), ("max_front", ctypes.c_int32),
-                ("n_fronts", ctypes.c_int32), ("n_tiles", ctypes.c_int32), ("n_mat", ctypes.c_int64),
-                ("level", NdLevel_t * MAX_LEVELS), ("fronts", _P), ("tiles", _P), ("piv_node", _P),
-                ("piv_src", _P), ("bnd_node", _P), ("bnd_src", _P), ("outside", _P), ("mat", _P)]
+                ("n_tiles", ctypes.c_int32), ("pad", ctypes.c_int32), ("n_mat", ctypes.c_int64),
+                ("level", NdLevel_t * MAX_LEVELS), ("tiles", _P), ("piv_node", _P), ("piv_src", _P),
+                ("bnd_node", _P), ("bnd_src", _P), ("outside", _P), ("mat", _P)]
 
 
-FRONT = np.dtype([("s", np.int32), ("b", np.int32), ("piv0", np.int32), ("bnd0", np.int32), ("ldf", np.int32),
-                  ("ldb", np.int32), ("mf", np.int64), ("mb", np.int64)], align=True)
+TILE = np.dtype([("mat", np.int64)] + [(k, np.int32) for k in ("n_in", "n_out", "ld", "o0", "piv0", "bnd0")])
 
 _lib.OTHER_DECLARED.update({"oec_nd_dissect"})
 
@@ -72,10 +76,40 @@ def dissect(ix, iy, max_depth, leaf=LEAF):
     return out
 
 
-# Model of a solve's time by which the levels are chosen (B200): a pass over
-# one level costs its dependent loads and a grid barrier, every front its share
-# of a warp's latency, and the blocks their bytes.
-PHASE_US, FRONT_US, GBS = 3.5, 1.0e-3, 6000.0
+# Model of a solve's time (B200, us) by which the levels and the tiles are
+# chosen.  A pass over one level costs a barrier.  A tile costs its chain of
+# dependent loads, a round of loads per GT inputs that its group of GT threads
+# gathers and one per 4 x GT pairs of outputs of its block; the pass takes as many
+# rounds of tiles as the groups need, and at least the time of the bytes that
+# the busiest SM reads.
+PHASE_US, TILE_US, GATHER_US, BLOCK_US, WARP_US, GBS_SM = 2.0, 2.0, 1.2, 0.8, 3.0, 44.0
+SMS = CTAS // 2
+
+
+def pass_plan(ins, outs):
+    """(modelled time, outputs per tile, threads per group) of one direction of
+    a level for fronts with `ins` inputs and `outs` outputs."""
+    if not outs.size or not outs.any():
+        return 0.0, 8, 512
+    n_in, n_out = int(ins.max()), int(outs.max())
+    best = None
+    for group, widths in ((512, (256, 128, 64, 32, 16, 8)), (128, (128, 64, 32, 16, 8))):
+        if group == 128 and n_in > QUARTER_IN:
+            continue
+        for w in widths:
+            tiles = int((-(-outs // w)).sum())
+            t = -(-tiles * group // (512 * CTAS)) * (TILE_US + GATHER_US * -(-n_in // group) +
+                                                     BLOCK_US * -(-n_in * w // (8 * group)))
+            t = max(t, -(-tiles // SMS) * n_in * min(w, n_out) * 8e-3 / GBS_SM)
+            if best is None or t < best[0]:
+                best = (t, w, group)
+    if n_in <= WARP_IN:
+        lanes = 32 if n_out > 32 else 16 if n_out > 16 else 8
+        t = -(-outs.size // (16 * CTAS)) * (WARP_US + BLOCK_US * -(-n_out // (2 * lanes)) * -(-n_in * lanes // 128))
+        t = max(t, -(-outs.size // SMS) * n_in * n_out * 8e-3 / GBS_SM)
+        if t < best[0]:
+            best = (t, 8, 32)
+    return best[0] + PHASE_US, best[1], best[2]
 
 
 def choose_levels(hid, dep, w, v, n):
@@ -102,32 +136,28 @@ def choose_levels(hid, dep, w, v, n):
             b = bnd[d]
             if s.max() > MAX_FRONT or b.max() > MAX_FRONT:
                 continue
-            s = s.astype(np.float64)
-            t = (1 if d == 0 else 2) * (PHASE_US + FRONT_US * np.count_nonzero(s)) + \
-                8e-3 * float((s * (s + 2.0 * b)).sum()) / GBS + best[d2][0]
+            ok = s > 0
+            t = pass_plan(s[ok], s[ok] + b[ok])[0] + best[d2][0]
+            if d:
+                t += pass_plan(b[ok], s[ok])[0]
             if cand is None or t < cand[0]:
                 cand = (t, [d] + best[d2][1], best[d2][2] + 1)
         best[d] = cand
     return None if best[0] is None else best[0][1]
 
 
-def _width(fronts_out, n_in, ctas):
-    """Outputs per tile of a level: 0 (a warp per front) when the fronts are
-    many and small, else the widest of 64 .. 8 that still gives every CTA a
-    tile."""
-    if n_in <= WARP_FRONT and fronts_out.size >= 4 * ctas:
-        return 0
-    for w in (64, 32, 16):
-        if int((-(-fronts_out // w)).sum()) >= 2 * ctas:
-            return w
-    return 8
+def host_inverse(A):
+    """Inverses of a stack of symmetric blocks (LinAlgError when one is singular)."""
+    X = np.linalg.inv(A)
+    return 0.5 * (X + X.transpose(0, 2, 1))
 
 
-def nd_host_arrays(a, inside, nx, n_nodes, ctas=296):
+def nd_host_arrays(a, inside, nx, n_nodes, inverse=host_inverse):
     """oec_nd_t's arrays for the CSC matrix `a` over the nodes `inside` of an
     extended grid nx nodes wide, or None when A is not a matrix of this form
     (couplings beyond grid neighbours, not symmetric, a singular front): the
-    level-scheduled factors take it, or refuse it."""
+    level-scheduled factors take it, or refuse it.  `inverse` replaces
+    host_inverse (the cubic part of the work on large grids)."""
     n = int(a.shape[0])
     inside = np.asarray(inside, np.int64)
     coo = a.tocoo()
@@ -236,8 +266,7 @@ def nd_host_arrays(a, inside, nx, n_nodes, ctas=296):
         A11 = F[:, :S, :S]
         for k, f in enumerate(fs):
             A11[k, np.arange(s[f], S), np.arange(s[f], S)] = 1.0
-        X = np.linalg.inv(A11)  # raises LinAlgError on a singular block
-        X = 0.5 * (X + X.transpose(0, 2, 1))
+        X = inverse(A11)
         A21 = F[:, S:, :S]
         G = A21 @ X
         C = F[:, S:, S:] - G @ A21.transpose(0, 2, 1) if B else None
@@ -262,12 +291,9 @@ def nd_host_arrays(a, inside, nx, n_nodes, ctas=296):
                 eliminate(part)
             except np.linalg.LinAlgError:
                 return None
-    out = {"n": n, "n_nodes": int(n_nodes), "n_bnd": int(bkey.size), "n_levels": K, "n_fronts": nf,
-           "max_front": int(max(s.max(), b.max())), "cuts": list(cuts), "level_of_front": flevel}
-    fr = np.zeros(nf, FRONT)
-    fr["s"], fr["b"], fr["piv0"], fr["bnd0"] = s, b, piv0[:-1], bnd0[:-1]
-    fr["ldf"], fr["ldb"], fr["mf"], fr["mb"] = ldf, ldb, mf[:-1], mf[:-1] + s * ldf
-    out["fronts"] = fr
+    out = {"n": n, "n_nodes": int(n_nodes), "n_bnd": int(bkey.size), "n_levels": K, "cuts": list(cuts),
+           "level_of_front": flevel, "s": s, "b": b, "piv0": piv0, "bnd0": bnd0, "ldf": ldf, "ldb": ldb,
+           "mf": mf[:-1], "mb": mf[:-1] + s * ldf}
     mask = np.ones(int(n_nodes), bool)
     mask[inside] = False
     out["outside"] = np.nonzero(mask)[0].astype(np.int32)
@@ -275,22 +301,33 @@ def nd_host_arrays(a, inside, nx, n_nodes, ctas=296):
     out["bnd_node"] = inside[bunk].astype(np.int32)
     out["piv_src"], out["bnd_src"] = np.ascontiguousarray(src[:n]), np.ascontiguousarray(src[n:])
     out["mat"] = mat
-    # tiles: (front, first output) per CTA, or (front, 0) per warp
     tiles, lv = [], []
-    count = 0
+    count, widest = 0, 16 * WARP_IN
     for k in range(K):
         fs = np.nonzero(flevel == k)[0]
         rec = {"has_children": int(np.any(np.isin(parent, fs)))}
-        for tag, outs, ins in (("fwd", s[fs] + b[fs], s[fs]), ("bwd", s[fs] if k else 0 * s[fs], b[fs])):
-            wd = _width(outs, int(ins.max()) if ins.size else 0, ctas)
-            per = np.where(outs > 0, 1, 0) if wd == 0 else -(-outs // wd)
-            t = np.zeros((int(per.sum()), 2), np.int32)
-            t[:, 0] = np.repeat(fs, per)
-            t[:, 1] = (np.arange(t.shape[0]) - np.repeat(np.cumsum(per) - per, per)) * wd
-            rec.update({tag + "_tile": count, tag + "_tiles": t.shape[0], tag + "_width": wd})
-            count += t.shape[0]
+        for tag in ("fwd", "bwd"):
+            fwd = tag == "fwd"
+            outs = s[fs] + b[fs] if fwd else s[fs] if k else 0 * s[fs]
+            ins = s[fs] if fwd else b[fs]
+            _, wd, group = pass_plan(ins, outs)
+            per = np.where(outs > 0, 1, 0) if group == 32 else -(-outs // wd)
+            t = np.zeros(int(per.sum()), TILE)
+            f = np.repeat(fs, per)
+            t["o0"] = (np.arange(t.size) - np.repeat(np.cumsum(per) - per, per)) * wd
+            t["n_in"] = np.repeat(ins, per)
+            left = np.repeat(outs, per) - t["o0"]
+            t["n_out"] = left if group == 32 else np.minimum(left, wd)
+            t["ld"] = (ldf if fwd else ldb)[f]
+            t["mat"] = (out["mf"] if fwd else out["mb"])[f] + t["o0"]
+            t["piv0"], t["bnd0"] = piv0[f], bnd0[f]
+            rec[tag] = {"tile": count, "tiles": t.size, "width": wd, "group": group}
+            count += t.size
+            if group > 32 and t.size:
+                widest = max(widest, int(t["n_in"].max()) * 512 // group)
             tiles.append(t)
         lv.append(rec)
+    out["max_front"] = -(-widest // 4) * 4
     out["tiles"] = np.ascontiguousarray(np.concatenate(tiles))
     out["level"] = lv
     return out
@@ -300,40 +337,52 @@ def nd_struct(a, ptr):
     """An Nd_t over the arrays of nd_host_arrays; ptr(name) gives the address
     of array `name` (host or device copy)."""
     t = Nd_t()
-    for k in ("n", "n_nodes", "n_bnd", "n_levels", "max_front", "n_fronts"):
+    for k in ("n", "n_nodes", "n_bnd", "n_levels", "max_front"):
         setattr(t, k, a[k])
-    t.n_outside, t.n_tiles, t.n_mat = a["outside"].size, a["tiles"].shape[0], a["mat"].size
+    t.n_outside, t.n_tiles, t.n_mat = a["outside"].size, a["tiles"].size, a["mat"].size
     for k, rec in enumerate(a["level"]):
-        for name, x in rec.items():
-            setattr(t.level[k], name, x)
-    for name in ("fronts", "tiles", "piv_node", "piv_src", "bnd_node", "bnd_src", "outside", "mat"):
+        t.level[k].has_children = rec["has_children"]
+        for tag in ("fwd", "bwd"):
+            for name, x in rec[tag].items():
+                setattr(getattr(t.level[k], tag), name, x)
+    for name in ("tiles", "piv_node", "piv_src", "bnd_node", "bnd_src", "outside", "mat"):
         setattr(t, name, ptr(name))
     return t
 
 
 def nd_solve_host(a, q):
-    """The device's solve restated with numpy: phi on all nodes."""
-    n = a["n"]
-    y, u, phi = np.zeros(n), np.zeros(a["n_bnd"] + 1), np.zeros(a["n_nodes"])
-    fr, mat = a["fronts"], a["mat"]
+    """The device's solve restated with numpy: phi on all nodes, tile by tile."""
+    y, u, phi = np.zeros(a["n"]), np.zeros(a["n_bnd"] + 1), np.zeros(a["n_nodes"])
+    mat = a["mat"]
 
     def gathered(src):
         return u[src].sum(1)  # -1 is the zero behind the last update
 
+    def product(t, v):
+        """The tile's outputs (its rows of the block start ld apart)."""
+        i = t["mat"] + np.arange(t["n_in"])[:, None] * t["ld"] + np.arange(t["n_out"])
+        return v @ mat[i]
+
+    def tiles_of(k, tag):
+        p = a["level"][k][tag]
+        return a["tiles"][p["tile"]:p["tile"] + p["tiles"]]
+
     for k in range(a["n_levels"] - 1, -1, -1):
-        for f in np.nonzero(a["level_of_front"] == k)[0]:
-            s, b, p0, b0 = (int(fr[f][x]) for x in ("s", "b", "piv0", "bnd0"))
-            v1 = q[a["piv_node"][p0:p0 + s]] + gathered(a["piv_src"][p0:p0 + s])
-            m = mat[fr[f]["mf"]:fr[f]["mf"] + s * fr[f]["ldf"]].reshape(s, -1)[:, :s + b]
-            o = v1 @ m
-            y[p0:p0 + s] = o[:s]
-            u[b0:b0 + b] = gathered(a["bnd_src"][b0:b0 + b]) - o[s:]
+        for t in tiles_of(k, "fwd"):
+            s, p0, o0 = int(t["n_in"]), int(t["piv0"]), int(t["o0"])
+            o = product(t, q[a["piv_node"][p0:p0 + s]] + gathered(a["piv_src"][p0:p0 + s]))
+            m = min(max(s - o0, 0), o.size)  # outputs that are pivots
+            y[p0 + o0:p0 + o0 + m] = o[:m]
+            e = int(t["bnd0"]) + np.arange(o0 + m - s, o0 + o.size - s)
+            u[e] = gathered(a["bnd_src"][e]) - o[m:]
     for k in range(a["n_levels"]):
-        for f in np.nonzero(a["level_of_front"] == k)[0]:
-            s, b, p0, b0 = (int(fr[f][x]) for x in ("s", "b", "piv0", "bnd0"))
-            x1 = y[p0:p0 + s].copy()
-            if b:
-                m = mat[fr[f]["mb"]:fr[f]["mb"] + b * fr[f]["ldb"]].reshape(b, -1)[:, :s]
-                x1 -= phi[a["bnd_node"][b0:b0 + b]] @ m
-            phi[a["piv_node"][p0:p0 + s]] = x1
+        if k == 0:
+            for t in tiles_of(0, "fwd"):
+                i = int(t["piv0"]) + int(t["o0"]) + np.arange(t["n_out"])
+                phi[a["piv_node"][i]] = y[i]
+            continue
+        for t in tiles_of(k, "bwd"):
+            i = int(t["piv0"]) + int(t["o0"]) + np.arange(t["n_out"])
+            e = int(t["bnd0"]) + np.arange(t["n_in"])
+            phi[a["piv_node"][i]] = y[i] - product(t, phi[a["bnd_node"][e]])
     return phi

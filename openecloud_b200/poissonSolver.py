@@ -31,7 +31,7 @@ from . import device as D
 from .constants import epsilon_0
 from .lu_setup import (LU_t, _level_lists, _levels, _np_ptr, assemble, choose_tail, factor,  # noqa: F401
                        level_lanes, lu_host_arrays, lu_struct, nd_lu_struct)
-from .nd_setup import nd_host_arrays, nd_struct
+from .nd_setup import host_inverse, nd_host_arrays, nd_struct
 
 
 class Stencil_t(ctypes.Structure):
@@ -206,6 +206,17 @@ def stencil_apply_host(meps, inside_mask, nx, x):
     return y
 
 
+def device_inverse(a):
+    """nd_setup.host_inverse on the device for blocks that are worth the copies
+    (a 1600 x 1600 one: 0.1 s on eight host cores, about 10 ms here)."""
+    if a.shape[1] < 64:
+        return host_inverse(a)
+    x, info = torch.linalg.inv_ex(D.to_device(a, torch.float64))
+    if int(info.abs().max().item()):
+        raise np.linalg.LinAlgError("singular front")
+    return D.to_numpy(0.5 * (x + x.mT))
+
+
 class PoissonSolver:
     """Reference: poissonSolver.pyx:33-67 (setup) and :83-98 (solve, getters)."""
 
@@ -373,13 +384,14 @@ class PoissonSolver:
         k["e_ptr"], k["e_idx"] = D.to_device(E.indptr, torch.int32), D.to_device(E.indices, torch.int32)
         k["e_val"] = D.to_device(E.data, torch.float64)
         nd = None if tail is not None else \
-            nd_host_arrays(self.systemMatrix, self.insidePointsInd, self.gridObj.getNxExt(), self.n_nodes)
+            nd_host_arrays(self.systemMatrix, self.insidePointsInd, self.gridObj.getNxExt(), self.n_nodes,
+                           device_inverse)
         if nd is None:
             self._factor_setup(tail)
             return
-        for name in ("tiles", "piv_node", "piv_src", "bnd_node", "bnd_src", "outside"):
+        for name in ("piv_node", "piv_src", "bnd_node", "bnd_src", "outside"):
             k[name] = D.to_device(nd[name], torch.int32)
-        k["fronts"] = D.to_device(nd["fronts"].view(np.uint8), torch.uint8)
+        k["tiles"] = D.to_device(nd["tiles"].view(np.uint8), torch.uint8)
         k["mat"] = D.to_device(nd["mat"], torch.float64)
         self._nd_t = nd_struct(nd, lambda name: D.ptr(k[name]))
         self._lu_t = nd_lu_struct(nd, self._nd_t)

@@ -36,8 +36,8 @@ def test_fronts_on_the_host(p, levels, monkeypatch):
     that costs nothing the tree is cut at (nearly) every depth."""
     from openecloud_b200 import nd_setup
     if levels == "many":
-        monkeypatch.setattr(nd_setup, "PHASE_US", 0.0)
-        monkeypatch.setattr(nd_setup, "FRONT_US", 0.0)
+        for k in ("PHASE_US", "TILE_US", "GATHER_US", "BLOCK_US", "WARP_US"):
+            monkeypatch.setattr(nd_setup, k, 0.0)
     g, a, inside, q, phi, tol = _case(p)
     h = nd_setup.nd_host_arrays(a, inside, g.getNxExt(), g.getNpExt())
     x = nd_setup.nd_solve_host(h, q)
@@ -71,8 +71,8 @@ def test_fronts_on_the_device(gpu, p, levels, monkeypatch):
     from openecloud_b200 import nd_setup
     from openecloud_b200.poissonSolver import PoissonSolver
     if levels == "many":
-        monkeypatch.setattr(nd_setup, "PHASE_US", 0.0)
-        monkeypatch.setattr(nd_setup, "FRONT_US", 0.0)
+        for k in ("PHASE_US", "TILE_US", "GATHER_US", "BLOCK_US", "WARP_US"):
+            monkeypatch.setattr(nd_setup, k, 0.0)
     g, a, inside, q, phi, tol = _case(p)
     ps = PoissonSolver(g)
     assert ps._lu_t.nd
