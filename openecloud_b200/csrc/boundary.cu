@@ -98,7 +98,7 @@ __global__ void k_mask_scatter(const uint32_t *__restrict__ mask, const int32_t 
 // The same index in one CTA for small stores (a few scan blocks): the words
 // are taken 1024 at a time with a running carry, so the three launches above
 // (count, block scan, scatter; ~3.5 us each at 1e5 particles) become one.
-constexpr int kSmallScanBlocks = 8;  // up to 8 * 1024 words = 262,144 particles
+constexpr int kSmallScanBlocks = 16;  // up to 16 * 1024 words = 524,288 particles
 
 __global__ void __launch_bounds__(kScanThreads)
     k_mask_index_small(const uint32_t *__restrict__ mask, const int32_t *count, int32_t *__restrict__ index,

@@ -4,7 +4,7 @@
 // and homoLoader (:41-72).  Two passes over the absorbed rows:
 //  pass 1: primary energy and incidence angle, elastic/rediffused/true yields
 //          and the number of secondaries drawn from P_n (:180-229);
-//  scan:   output offsets of each absorbed particle's secondaries;
+//          summed per 32 rows;
 //  emit:   energies (single secondary: elastic/rediffused/true split;
 //          several: the joint energy split through I_x and P inverses,
 //          :232-278) and cos-law directions about the wall normal (:280-302).
@@ -42,6 +42,7 @@ __device__ __forceinline__ double clip(double x, double lo, double hi) {
 }
 
 constexpr int kSlots = 10;
+constexpr int kTileRows = 32;  // rows whose secondaries pass 1 sums
 constexpr int kClasses = kSlots * (kSlots + 1) / 2;  // (n, k), k < n: n (n - 1) / 2 + k
 
 // The constants of the inverses of k_furman_emit, by (n, k).
@@ -57,7 +58,10 @@ __global__ void __launch_bounds__(128)
     k_furman_pass1(oec_furman_t f, const double *__restrict__ rows, const double *__restrict__ normals,
                    const int32_t *n_abs, int cap, const int32_t *__restrict__ ids, uint2 key, uint32_t step,
                    const int32_t *step_dev, const double *__restrict__ replay, Rec *__restrict__ rec,
-                   int32_t *__restrict__ nsec, oec_status_t *status, int row_blocks, SplitConst *__restrict__ consts) {
+                   int32_t *__restrict__ tile_sum, oec_status_t *status, int row_blocks,
+                   SplitConst *__restrict__ consts) {
+    const int na = min(*n_abs, cap);
+    if (na <= 0) return;
     if ((int)blockIdx.x >= row_blocks) {
         const int c = blockIdx.x - row_blocks;
         int n = 1, k;
@@ -76,7 +80,6 @@ __global__ void __launch_bounds__(128)
             sf::beta_const(P * (n - k - 1), P, consts->beta[(n - 1) * (n - 2) / 2 + k]);
         return;
     }
-    int na = min(*n_abs, cap);
     const double eFactor = 0.5 * f.particle_mass / 1.602176565e-19;
     int wd = 0, wt = 0;
     __shared__ double lfac[11];  // lgamma(j + 1), j <= m <= 10
@@ -84,16 +87,16 @@ __global__ void __launch_bounds__(128)
     if (threadIdx.x <= f.m) lfac[threadIdx.x] = sf::lgam((double)threadIdx.x + 1.0);
     __syncthreads();
     int skipped = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < na; i += row_blocks * blockDim.x) {
+    // the number of secondaries of row i
+    auto row = [&](int i) -> int {
         const double *r = rows + 6 * (int64_t)i;
         const double n0 = normals[2 * i], n1 = normals[2 * i + 1];
         double v0 = sqrt(r[2] * r[2] + r[3] * r[3] + r[4] * r[4]);
         double e0 = eFactor * v0 * v0;
         if (!row_emits(r, e0, n0, n1)) {
             rec[i] = Rec{0., 0., 0., 1., 0};
-            nsec[i] = 0;
             ++skipped;
-            continue;
+            return 0;
         }
         double th = acos((r[2] * n0 + r[3] * n1) / v0);
         if (th > 0.5 * sf::kPi) th = sf::kPi - th;
@@ -146,7 +149,12 @@ __global__ void __launch_bounds__(128)
             }
         }
         rec[i] = Rec{e0, dE, dR, pN1, n};
-        nsec[i] = n;
+        return n;
+    };
+    // a warp takes kTileRows consecutive rows and leaves their sum for the next kernel's places
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; (i & ~31) < na; i += row_blocks * blockDim.x) {
+        const int sum = __reduce_add_sync(kFullMask, i < na ? row(i) : 0);
+        if ((i & 31) == 0) tile_sum[i >> 5] = sum;
     }
     if (wd) atomicAdd(&status->warn_derm, wd);
     if (wt) atomicAdd(&status->warn_tsprime, wt);
@@ -179,23 +187,52 @@ __device__ __forceinline__ void put_secondary(const double *r, double n0, double
 //
 // The inverses are most of the work.  They differ in their branch and their
 // length by (n, k) above all, and most of a row's kSlots slots are empty, so a
-// CTA takes a chunk of rows, sorts its secondaries by (n, k) in shared memory and
-// works them off in that order, a warp taking the next 32 when it is free: the
-// lanes of a warp run the same branch of the same function, with the
-// constants of (n, k) from pass 1 (specfun.cuh).  Which lane takes which
+// CTA takes a chunk of rows, sorts its secondaries by function and (n, k) in
+// shared memory and works them off in that order, a warp taking the next (at
+// most) 32 of one function when it is free: the lanes of a warp run the same
+// branch of the same function, with the constants of (n, k) from pass 1
+// (specfun.cuh), and with few rows the functions run side by side.  Which lane takes which
 // does not enter its value.  106,457 absorbed rows of 200 eV electrons (179,048
 // secondaries) on a B200: 3340 us for a thread per (row, slot) with the plain
 // inverses and a thread per row for the directions, 132 us this way; 250 secondaries
 // (one buildup step): 40 us, the latency of one inverse.
 constexpr int kSplitT = 256, kSplitRows = 1024;
+constexpr int kKinds = 9;  // lone, gamma, and the kinds of sf::BetaConst
 
 struct SplitShared {
     SplitConst c;
-    int count[kClasses + 1];                // secondaries, then the place after the last one put
-    int next[2];                            // secondaries handed out to the warps, per phase
+    int first[kSplitRows];                  // a row's first secondary, from the chunk's first
+    int warp_sum[2][kSplitT / 32];
+    unsigned char kind[kClasses];           // the function a class is inverted by
+    unsigned char rank[kClasses];           // a class's place in the order of the kinds
+    int kind_first[kKinds + 1];             // first rank of a kind
+    int count[kClasses + 1];                // per rank: secondaries, then the place after the last one put
+    int batch[kKinds][3];                   // per kind: batches before it, first and last place
+    int next[2];                            // batches handed out to the warps, per phase
     unsigned char nsec[kSplitRows];
     unsigned task[kSplitRows * kSlots];     // row in the chunk | n << 16 | k << 24
 };
+
+// The next batch of this warp, at most 32 secondaries of one kind: this lane's
+// place, or -1.  False when none are left.
+__device__ __forceinline__ bool next_batch(SplitShared &sh, int *t) {
+    int first = -1, last = 0;
+    if ((threadIdx.x & 31) == 0) {
+        const int b = atomicAdd(&sh.next[0], 1);
+        for (int g = 0; g < kKinds; ++g) {
+            const int k = b - sh.batch[g][0], at = sh.batch[g][1] + 32 * k;
+            if (k >= 0 && at < sh.batch[g][2]) {
+                first = at;
+                last = min(at + 32, sh.batch[g][2]);
+            }
+        }
+    }
+    first = __shfl_sync(kFullMask, first, 0);
+    last = __shfl_sync(kFullMask, last, 0);
+    *t = first + (int)(threadIdx.x & 31);
+    if (*t >= last) *t = -1;
+    return first >= 0;
+}
 
 // The next 32 secondaries for this warp; this lane's one, or -1.  False when
 // none are left.
@@ -213,13 +250,15 @@ __global__ void __launch_bounds__(kSplitT)
                   const int32_t *n_abs, int cap, const int32_t *__restrict__ ids, uint2 key, uint32_t step,
                   const int32_t *step_dev, const double *__restrict__ replay, const Rec *__restrict__ rec,
                   const SplitConst *__restrict__ consts, double *__restrict__ split,
-                  const int32_t *__restrict__ offset, double *__restrict__ out, int out_cap, oec_status_t *status) {
+                  const int32_t *__restrict__ tile_sum, double *__restrict__ out, int out_cap, int32_t *n_out,
+                  oec_status_t *status) {
     extern __shared__ __align__(16) unsigned char split_smem[];
     SplitShared &sh = *reinterpret_cast<SplitShared *>(split_smem);
     const int na = min(*n_abs, cap);
     // rows per chunk: all CTAs busy before the chunks reach full size
     const int per = (na + (int)gridDim.x - 1) / (int)gridDim.x;
     const int chunk = min(kSplitRows, max(32, (per + 31) & ~31));
+    if (na <= 0 && blockIdx.x == 0 && threadIdx.x == 0) *n_out = 0;
     if ((int)blockIdx.x * chunk >= na) return;
     const uint32_t st = step + (step_dev ? (uint32_t)*step_dev : 0u);
     const int tid = threadIdx.x;
@@ -229,17 +268,67 @@ __global__ void __launch_bounds__(kSplitT)
     for (int i = tid; i < (int)(sizeof(SplitConst) / sizeof(int4)); i += kSplitT)
         reinterpret_cast<int4 *>(&sh.c)[i] = __ldg(reinterpret_cast<const int4 *>(consts) + i);
     int dropped = 0;
+    const int lane = tid & 31, warp = tid >> 5;
+    __syncthreads();
+    if (tid < kClasses) {
+        int n = 1;
+        while (n * (n + 1) / 2 <= tid) ++n;
+        const int k = tid - n * (n - 1) / 2;
+        sh.kind[tid] = (unsigned char)(n == 1 ? 0 : k == n - 1 ? 1 : 2 + sh.c.beta[(n - 1) * (n - 2) / 2 + k].kind);
+    }
+    __syncthreads();
+    if (tid < kClasses || (tid >= 64 && tid <= 64 + kKinds)) {
+        const int key = tid < kClasses ? sh.kind[tid] * 64 + tid : (tid - 64) * 64;
+        int r = 0;
+        for (int c = 0; c < kClasses; ++c) r += sh.kind[c] * 64 + c < key ? 1 : 0;
+        if (tid < kClasses)
+            sh.rank[tid] = (unsigned char)r;
+        else
+            sh.kind_first[tid - 64] = r;
+    }
+    __syncthreads();
+    int before = 0, summed = 0;  // secondaries of the rows before the chunk; tiles in `before`
     for (int r0 = blockIdx.x * chunk; r0 < na; r0 += gridDim.x * chunk) {
         const int nrows = min(chunk, na - r0);
         for (int c = tid; c <= kClasses; c += kSplitT) sh.count[c] = 0;
         if (tid < 2) sh.next[tid] = 0;
         __syncthreads();
-        for (int r = tid; r < nrows; r += kSplitT) {
-            const int n = rec[r0 + r].nsec;
-            sh.nsec[r] = (unsigned char)n;
-            for (int k = 0; k < n; ++k) atomicAdd(&sh.count[n * (n - 1) / 2 + k], 1);
+        // a thread's kPer consecutive rows: their counts and, by a scan over the
+        // CTA, the place of their first secondaries; with them the sum of the
+        // tiles between the last chunk and this one
+        constexpr int kPer = kSplitRows / kSplitT;
+        int cnt[kPer], mine = 0, tiles = 0;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const int r = tid * kPer + j;
+            cnt[j] = r < nrows ? rec[r0 + r].nsec : 0;
+            sh.nsec[r] = (unsigned char)cnt[j];
+            for (int k = 0; k < cnt[j]; ++k) atomicAdd(&sh.count[sh.rank[cnt[j] * (cnt[j] - 1) / 2 + k]], 1);
+            mine += cnt[j];
         }
+        for (int q = summed + tid; q < r0 / kTileRows; q += kSplitT) tiles += tile_sum[q];
+        summed = r0 / kTileRows;
+        tiles = __reduce_add_sync(kFullMask, tiles);
+        int scan = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kFullMask, scan, o);
+            if (lane >= o) scan += y;
+        }
+        if (lane == 31) sh.warp_sum[0][warp] = scan;
+        if (lane == 0) sh.warp_sum[1][warp] = tiles;
         __syncthreads();
+        int at = scan - mine;
+        for (int w = 0; w < kSplitT / 32; ++w) {
+            if (w < warp) at += sh.warp_sum[0][w];
+            before += sh.warp_sum[1][w];
+        }
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            sh.first[tid * kPer + j] = at;
+            at += cnt[j];
+        }
+        if (r0 + nrows == na && tid == kSplitT - 1) *n_out = before + at;
         if (tid < 32) {  // exclusive scan of the counts by one warp
             int carry = 0;
             for (int c0 = 0; c0 <= kClasses; c0 += 32) {
@@ -256,15 +345,23 @@ __global__ void __launch_bounds__(kSplitT)
         }
         __syncthreads();
         const int total = sh.count[kClasses], lone = sh.count[1];  // class 0 comes first
+        if (tid == 0)
+            for (int g = 0, nb = 0; g < kKinds; ++g) {
+                const int a = sh.count[sh.kind_first[g]], b = sh.count[sh.kind_first[g + 1]];
+                sh.batch[g][0] = nb;
+                sh.batch[g][1] = a;
+                sh.batch[g][2] = b;
+                nb += (b - a + 31) / 32;
+            }
         __syncthreads();
         for (int r = tid; r < nrows; r += kSplitT) {
             const int n = sh.nsec[r];
-            for (int k = 0; k < n; ++k) sh.task[atomicAdd(&sh.count[n * (n - 1) / 2 + k], 1)] = r | n << 16 | k << 24;
+            for (int k = 0; k < n; ++k) sh.task[atomicAdd(&sh.count[sh.rank[n * (n - 1) / 2 + k]], 1)] = r | n << 16 | k << 24;
         }
         __syncthreads();
         // the inverses; a lone secondary is finished here
         int t;
-        while (next_task(&sh.next[0], total, &t)) {
+        while (next_batch(sh, &t)) {
             if (t < 0) continue;
             const unsigned w = sh.task[t];
             const int row = r0 + (int)(w & 0xffff), n = (w >> 16) & 0xff, k = w >> 24;
@@ -296,7 +393,7 @@ __global__ void __launch_bounds__(kSplitT)
             } else {
                 e = f.epsN[0] * sf::gammaincinv_t(G, dr.next() * sf::gammainc_of(G, e0 / f.epsN[0]));
             }
-            const int o = offset[row];
+            const int o = before + sh.first[row - r0];
             if (o < out_cap)
                 put_secondary(rows + 6 * (int64_t)row, normals[2 * row], normals[2 * row + 1], sqrt(eFactorInv * e), dr,
                               out + 6 * (int64_t)o);
@@ -309,7 +406,7 @@ __global__ void __launch_bounds__(kSplitT)
             if (t < 0) continue;
             const unsigned w = sh.task[lone + t];
             const int row = r0 + (int)(w & 0xffff), n = (w >> 16) & 0xff, k = w >> 24;
-            const int o = offset[row] + k;
+            const int o = before + sh.first[row - r0] + k;
             if (o >= out_cap) {
                 ++dropped;
                 continue;
@@ -325,6 +422,7 @@ __global__ void __launch_bounds__(kSplitT)
                           sqrt(eFactorInv * (f.epsN[n - 1] * e)), dr, out + 6 * (int64_t)o);
         }
         __syncthreads();
+        // the rows of this chunk are part of the tiles that the next one sums
     }
     if (dropped) atomicAdd(&status->n_capacity_drop, dropped);
 }
@@ -645,24 +743,17 @@ extern "C" int oec_furman_emit(const oec_furman_t *params, const double *rows_de
         return OEC_ERR_INVALID;
     if (cap > kMaxAbsorbedRows) return OEC_ERR_INVALID;
     cudaStream_t s = as_stream(stream);
-    // work layout: SplitConst | Rec[cap] | split[cap * kSlots] (f64) | nsec[cap] | offset[cap] |
-    // partial[scan_blocks(cap)]
+    // work layout: SplitConst | Rec[cap] | split[cap * kSlots] (f64) | tile_sum[cap / kTileRows]
     char *w = static_cast<char *>(work_dev);
     SplitConst *consts = reinterpret_cast<SplitConst *>(w);
     Rec *rec = reinterpret_cast<Rec *>(w + sizeof(SplitConst));
     double *split = reinterpret_cast<double *>(rec + cap);
-    int32_t *nsec = reinterpret_cast<int32_t *>(split + (size_t)cap * kSlots);
-    int32_t *off = nsec + cap;
-    int *partial = off + cap;
+    int32_t *tile_sum = reinterpret_cast<int32_t *>(split + (size_t)cap * kSlots);
     uint2 key = make_uint2((uint32_t)seed, (uint32_t)(seed >> 32));
     const int g = persistent_grid((cap + 127) / 128, 8);
     k_furman_pass1<<<g + kClasses + kSlots, 128, 0, s>>>(*params, rows_dev, normals_dev, n_abs_dev, cap, ids_dev, key, step,
-                                                step_dev, replay_uniforms_dev, rec, nsec, status_dev, g, consts);
-    if (cap > 0) {
-        scan_counts(nsec, n_abs_dev, cap, off, partial, n_out_dev, s);
-    } else {
-        OEC_CUDA_TRY(cudaMemsetAsync(n_out_dev, 0, sizeof(int32_t), s));
-    }
+                                                         step_dev, replay_uniforms_dev, rec, tile_sum, status_dev, g,
+                                                         consts);
     static std::atomic<int> attr[kMaxDevices];
     const int ok = per_device_cached(attr, [] {
         return cudaFuncSetAttribute(k_furman_emit, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -672,8 +763,8 @@ extern "C" int oec_furman_emit(const oec_furman_t *params, const double *rows_de
     });
     if (!ok) return OEC_ERR_CUDA;
     k_furman_emit<<<persistent_grid((cap + 31) / 32, 2), kSplitT, sizeof(SplitShared), s>>>(
-        *params, rows_dev, normals_dev, n_abs_dev, cap, ids_dev, key, step, step_dev, replay_uniforms_dev, rec,
-        consts, split, off, out_rows_dev, out_cap, status_dev);
+        *params, rows_dev, normals_dev, n_abs_dev, cap, ids_dev, key, step, step_dev, replay_uniforms_dev, rec, consts,
+        split, tile_sum, out_rows_dev, out_cap, n_out_dev, status_dev);
     OEC_LAUNCH_CHECK();
     return OEC_OK;
 }
@@ -717,8 +808,8 @@ extern "C" int64_t oec_secelec_work_bytes(int32_t cap) {
 
 extern "C" int64_t oec_furman_work_bytes(int32_t cap) {
     if (cap < 0 || cap > kMaxAbsorbedRows) return -1;
-    return (int64_t)sizeof(SplitConst) + (int64_t)sizeof(Rec) * cap + (int64_t)sizeof(double) * kSlots * cap + 2 * sizeof(int32_t) * (int64_t)cap +
-           sizeof(int) * (int64_t)scan_blocks(cap) + 256;
+    return (int64_t)sizeof(SplitConst) + (int64_t)sizeof(Rec) * cap + (int64_t)sizeof(double) * kSlots * cap +
+           sizeof(int32_t) * ((int64_t)cap / kTileRows + 1) + 256;
 }
 
 extern "C" int oec_homo_load(const oec_grid_t *grid, const oec_boundary_t *boundary, oec_particles_t *p, int64_t n,
