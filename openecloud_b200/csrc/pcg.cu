@@ -205,6 +205,11 @@ __global__ void __launch_bounds__(kT) k_scale32(int G, const double *__restrict_
     for (int i = blockIdx.x * kT + threadIdx.x; i < G; i += gridDim.x * kT) r[i] = (float)(r64[i] * s);
 }
 
+// The work area is the caller's, so its vectors may lie at any float.
+__device__ __forceinline__ bool aligned16(const void *a, const void *b) {
+    return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15u) == 0;
+}
+
 // q = A32 p; acc[slot].pq += p.q.  First kernel of an inner iteration: it
 // disarms the loop, which only the convergence check re-arms.
 __global__ void __launch_bounds__(kT) k_apply32(int nx, int G, const float *__restrict__ ex,
@@ -246,7 +251,23 @@ __global__ void __launch_bounds__(kT) k_update32(int G, const float *__restrict_
     }
     const float alpha = (float)(rzv / pq);
     double rr = 0.0, rzn = 0.0, zq = 0.0;
-    for (int i = blockIdx.x * kT + threadIdx.x; i < G; i += gridDim.x * kT) {
+    // 16 bytes a load (10.5 -> 9.5 us at 1024^2); the rest, or all of it, one by one
+    const int n4 = precond > OEC_PRECOND_JACOBI && aligned16(p, q) && aligned16(d, r) ? G >> 2 : 0;
+    for (int k = blockIdx.x * kT + threadIdx.x; k < n4; k += gridDim.x * kT) {
+        const float4 pv = reinterpret_cast<const float4 *>(p)[k], qv = reinterpret_cast<const float4 *>(q)[k];
+        float4 dv = reinterpret_cast<float4 *>(d)[k], rv = reinterpret_cast<float4 *>(r)[k];
+        dv = make_float4(fmaf(alpha, pv.x, dv.x), fmaf(alpha, pv.y, dv.y), fmaf(alpha, pv.z, dv.z),
+                         fmaf(alpha, pv.w, dv.w));
+        rv = make_float4(fmaf(-alpha, qv.x, rv.x), fmaf(-alpha, qv.y, rv.y), fmaf(-alpha, qv.z, rv.z),
+                         fmaf(-alpha, qv.w, rv.w));
+        reinterpret_cast<float4 *>(d)[k] = dv;
+        reinterpret_cast<float4 *>(r)[k] = rv;
+        rr += (double)rv.x * (double)rv.x;
+        rr += (double)rv.y * (double)rv.y;
+        rr += (double)rv.z * (double)rv.z;
+        rr += (double)rv.w * (double)rv.w;
+    }
+    for (int i = 4 * n4 + blockIdx.x * kT + threadIdx.x; i < G; i += gridDim.x * kT) {
         const float qi = q[i];
         d[i] = fmaf(alpha, p[i], d[i]);
         const float ri = fmaf(-alpha, qi, r[i]);
@@ -305,7 +326,13 @@ __global__ void __launch_bounds__(kT) k_direction32(int G, const float *__restri
     if (!isfinite(b)) b = 0.0;
     const float beta = (float)b;
     if (isfinite(a->rr) && isfinite(rz) && a->pq > 0.0) {
-        for (int i = blockIdx.x * kT + threadIdx.x; i < G; i += gridDim.x * kT) p[i] = fmaf(beta, p[i], z[i]);
+        const int n4 = aligned16(p, z) ? G >> 2 : 0;
+        for (int k = blockIdx.x * kT + threadIdx.x; k < n4; k += gridDim.x * kT) {
+            const float4 pv = reinterpret_cast<const float4 *>(p)[k], zv = reinterpret_cast<const float4 *>(z)[k];
+            reinterpret_cast<float4 *>(p)[k] = make_float4(fmaf(beta, pv.x, zv.x), fmaf(beta, pv.y, zv.y),
+                                                           fmaf(beta, pv.z, zv.z), fmaf(beta, pv.w, zv.w));
+        }
+        for (int i = 4 * n4 + blockIdx.x * kT + threadIdx.x; i < G; i += gridDim.x * kT) p[i] = fmaf(beta, p[i], z[i]);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         // a breakdown (rr NaN) propagates: the next update sees rz NaN
@@ -472,39 +499,69 @@ struct MgT {
     const float *ex, *ey, *leak, *dinv;
 };
 
-// (A v) at fine node (gx, gy), i = gy * nx + gx, from a shared tile s with
-// row stride S whose entry (sy, sx) holds node (gx, gy): leak v_i + sum over
-// the 4 edges of w (v_i - v_j).  Nodes beyond the grid hold 0 in s.
+// What a tile works on, in shared memory: the operator and the right-hand
+// side on the tile grown by two nodes (zero beyond the grid), loaded in one
+// round of independent loads.  The sweeps then touch no global memory; when
+// they read the operator themselves a tile was four dependent rounds long
+// (V-cycle 1024^2 86 -> 75 us, 512^2 56 -> 48 us, 128^2 35 -> 31 us).
+constexpr int kTW = kTX + 4, kTile1 = (kTY + 4) * kTW, kTW2 = kTX + 2, kTile2 = (kTY + 2) * kTW2;
+struct TileMem {
+    float b[kTile1], d[kTile1], ex[kTile1], ey[kTile1], lk[kTile1];
+    float s1[kTile1], s2[kTile2];
+};
+
+// Loads the tile at (x0, y0); start(i, gx, gy, d, b) gives s1 on inside nodes.
+template <class F>
+__device__ __forceinline__ void tile_load(TileMem &T, const MgT &L, const float *b, int x0, int y0, F start) {
+#pragma unroll
+    for (int j = 0; j < (kTile1 + kT - 1) / kT; ++j) {
+        const int e = threadIdx.x + j * kT;
+        if (e < kTile1) {
+            const int ly = e / kTW, lx = e - ly * kTW;
+            const int gx = x0 + lx - 2, gy = y0 + ly - 2;
+            float bv = 0.f, d = 0.f, ex = 0.f, ey = 0.f, lk = 0.f, v = 0.f;
+            if (gx >= 0 && gy >= 0 && gx < L.nx && gy < L.ny) {
+                const int i = gy * L.nx + gx;
+                d = L.dinv[i];
+                ex = L.ex[i];
+                ey = L.ey[i];
+                if (L.leak) lk = L.leak[i];
+                bv = b[i];
+                v = start(i, gx, gy, d, bv);
+            }
+            T.b[e] = bv;
+            T.d[e] = d;
+            T.ex[e] = ex;
+            T.ey[e] = ey;
+            T.lk[e] = lk;
+            T.s1[e] = v;
+        }
+    }
+}
+
+// (A v) at node (gx, gy): entry e of the tile's operator, entry f of v with
+// row stride S: leak v_i + sum over the 4 edges of w (v_i - v_j).
 template <int S>
-__device__ __forceinline__ float tile_apply(const MgT &L, int i, int gx, int gy, const float *s, int sy, int sx) {
-    const float c = s[sy * S + sx];
-    float y = L.leak ? L.leak[i] * c : 0.f;
-    y += L.ex[i] * (c - s[sy * S + sx + 1]);
-    if (gx > 0) y += L.ex[i - 1] * (c - s[sy * S + sx - 1]);
-    y += L.ey[i] * (c - s[(sy + 1) * S + sx]);
-    if (gy > 0) y += L.ey[i - L.nx] * (c - s[(sy - 1) * S + sx]);
+__device__ __forceinline__ float tile_apply(const TileMem &T, bool leak, int e, int gx, int gy, const float *v, int f) {
+    const float c = v[f];
+    float y = leak ? T.lk[e] * c : 0.f;
+    y += T.ex[e] * (c - v[f + 1]);
+    if (gx > 0) y += T.ex[e - 1] * (c - v[f - 1]);
+    y += T.ey[e] * (c - v[f + S]);
+    if (gy > 0) y += T.ey[e - kTW] * (c - v[f - S]);
     return y;
 }
 
-// One damped-Jacobi sweep on the tile grown by `grow` (1 or 0) from the
-// values in `src` (tile grown by grow + 1): dst = v + w D^-1 (b - A v).
-template <int SS, int DS, int GROW>
-__device__ __forceinline__ void tile_sweep(const MgT &L, float om, const float *__restrict__ b, int x0, int y0,
-                                           const float *src, float *dst) {
-    constexpr int W = kTX + 2 * GROW, H = kTY + 2 * GROW;
-    for (int e = threadIdx.x; e < W * H; e += blockDim.x) {
-        const int ly = e / W, lx = e - ly * W;
-        const int gx = x0 + lx - GROW, gy = y0 + ly - GROW;
+// First damped-Jacobi sweep, on the tile grown by one node: s2 = s1 + w D^-1
+// (b - A s1).
+__device__ __forceinline__ void tile_sweep(TileMem &T, bool leak, float om, int x0, int y0) {
+    for (int k = threadIdx.x; k < kTile2; k += kT) {
+        const int ly = k / kTW2, lx = k - ly * kTW2, e = (ly + 1) * kTW + lx + 1;
+        const float d = T.d[e];
         float v = 0.f;
-        if (gx >= 0 && gy >= 0 && gx < L.nx && gy < L.ny) {
-            const int i = gy * L.nx + gx;
-            const float d = L.dinv[i];
-            if (d != 0.f) {
-                const float c = src[(ly + 1) * SS + lx + 1];
-                v = c + om * d * (b[i] - tile_apply<SS>(L, i, gx, gy, src, ly + 1, lx + 1));
-            }
-        }
-        dst[ly * DS + lx] = v;
+        if (d != 0.f)
+            v = T.s1[e] + om * d * (T.b[e] - tile_apply<kTW>(T, leak, e, x0 + lx - 1, y0 + ly - 1, T.s1, e));
+        T.s2[k] = v;
     }
 }
 
@@ -512,37 +569,23 @@ __device__ __forceinline__ void tile_sweep(const MgT &L, float om, const float *
 // coarse right-hand side bc[I] = sum over the inside children of (b - A x).
 // Node (r, c) belongs to coarse node (r >> SY, c >> SX).
 template <int SX, int SY>
-__global__ void __launch_bounds__(kT) k_mg_down(MgT L, float om, const float *__restrict__ b, float *__restrict__ x,
-                                                float *__restrict__ bc, int cnx, int cny) {
-    pdl_wait();
-    pdl_launch();
-    __shared__ float s1[(kTY + 4) * (kTX + 4)];
-    __shared__ float s2[(kTY + 2) * (kTX + 2)];
-    const int x0 = blockIdx.x * kTX, y0 = blockIdx.y * kTY;
-    for (int e = threadIdx.x; e < (kTY + 4) * (kTX + 4); e += kT) {
-        const int ly = e / (kTX + 4), lx = e - ly * (kTX + 4);
-        const int gx = x0 + lx - 2, gy = y0 + ly - 2;
-        float v = 0.f;
-        if (gx >= 0 && gy >= 0 && gx < L.nx && gy < L.ny) {
-            const int i = gy * L.nx + gx;
-            v = om * L.dinv[i] * b[i];
-        }
-        s1[e] = v;
-    }
+__device__ __forceinline__ void mg_down_tile(const MgT &L, float om, const float *b, float *x, float *bc, int cnx, int cny,
+                                             int x0, int y0, TileMem &T) {
+    const bool leak = L.leak != nullptr;
+    tile_load(T, L, b, x0, y0, [&](int, int, int, float d, float bv) { return om * d * bv; });
     __syncthreads();
-    tile_sweep<kTX + 4, kTX + 2, 1>(L, om, b, x0, y0, s1, s2);
+    tile_sweep(T, leak, om, x0, y0);
     __syncthreads();
-    float *res = s1;  // [kTY][kTX]
-    for (int e = threadIdx.x; e < kTY * kTX; e += kT) {
-        const int ly = e / kTX, lx = e - ly * kTX;
+    float *res = T.s1;  // [kTY][kTX]
+    for (int k = threadIdx.x; k < kTY * kTX; k += kT) {
+        const int ly = k / kTX, lx = k - ly * kTX, e = (ly + 2) * kTW + lx + 2, f = (ly + 1) * kTW2 + lx + 1;
         const int gx = x0 + lx, gy = y0 + ly;
         float v = 0.f;
         if (gx < L.nx && gy < L.ny) {
-            const int i = gy * L.nx + gx;
-            x[i] = s2[(ly + 1) * (kTX + 2) + lx + 1];
-            if (L.dinv[i] != 0.f) v = b[i] - tile_apply<kTX + 2>(L, i, gx, gy, s2, ly + 1, lx + 1);
+            x[gy * L.nx + gx] = T.s2[f];
+            if (T.d[e] != 0.f) v = T.b[e] - tile_apply<kTW2>(T, leak, e, gx, gy, T.s2, f);
         }
-        res[e] = v;
+        res[k] = v;
     }
     __syncthreads();
     constexpr int CW = kTX >> SX, CH = kTY >> SY;
@@ -559,9 +602,47 @@ __global__ void __launch_bounds__(kT) k_mg_down(MgT L, float om, const float *__
     }
 }
 
+template <int SX, int SY>
+__global__ void __launch_bounds__(kT) k_mg_down(MgT L, float om, const float *__restrict__ b, float *__restrict__ x,
+                                                float *__restrict__ bc, int cnx, int cny) {
+    pdl_wait();
+    pdl_launch();
+    __shared__ TileMem T;
+    mg_down_tile<SX, SY>(L, om, b, x, bc, cnx, cny, blockIdx.x * kTX, blockIdx.y * kTY, T);
+}
+
 // Up: t = x + scale * yc[parent] (inside nodes), two sweeps, result to out.
-// With acc, also acc[slot].rzn += b.out and acc[slot].zq += out.q (b is the
-// level-0 residual r, out the preconditioned z).
+// With q, also *rz += b.out and *zq += out.q (b is the level-0 residual r,
+// out the preconditioned z).
+template <int SX, int SY>
+__device__ __forceinline__ void mg_up_tile(const MgT &L, float om, float scale, const float *b, const float *x,
+                                           const float *yc, int cnx, float *out, const float *q, double *rz, double *zq,
+                                           int x0, int y0, TileMem &T) {
+    const bool leak = L.leak != nullptr;
+    tile_load(T, L, b, x0, y0, [&](int i, int gx, int gy, float d, float) {
+        const float v = x[i] + scale * yc[(gy >> SY) * cnx + (gx >> SX)];
+        return d != 0.f ? v : 0.f;
+    });
+    __syncthreads();
+    tile_sweep(T, leak, om, x0, y0);
+    __syncthreads();
+    for (int k = threadIdx.x; k < kTY * kTX; k += kT) {
+        const int ly = k / kTX, lx = k - ly * kTX, e = (ly + 2) * kTW + lx + 2, f = (ly + 1) * kTW2 + lx + 1;
+        const int gx = x0 + lx, gy = y0 + ly;
+        if (gx < L.nx && gy < L.ny) {
+            const int i = gy * L.nx + gx;
+            const float d = T.d[e], bi = T.b[e];
+            float v = 0.f;
+            if (d != 0.f) v = T.s2[f] + om * d * (bi - tile_apply<kTW2>(T, leak, e, gx, gy, T.s2, f));
+            out[i] = v;
+            if (q) {
+                *rz += (double)bi * (double)v;
+                *zq += (double)v * (double)q[i];
+            }
+        }
+    }
+}
+
 template <int SX, int SY>
 __global__ void __launch_bounds__(kT) k_mg_up(MgT L, float om, float scale, const float *__restrict__ b,
                                               const float *__restrict__ x, const float *__restrict__ yc, int cnx,
@@ -569,41 +650,10 @@ __global__ void __launch_bounds__(kT) k_mg_up(MgT L, float om, float scale, cons
                                               const Ctl *ctl) {
     pdl_wait();
     pdl_launch();
-    __shared__ float s1[(kTY + 4) * (kTX + 4)];
-    __shared__ float s2[(kTY + 2) * (kTX + 2)];
-    const int x0 = blockIdx.x * kTX, y0 = blockIdx.y * kTY;
-    for (int e = threadIdx.x; e < (kTY + 4) * (kTX + 4); e += kT) {
-        const int ly = e / (kTX + 4), lx = e - ly * (kTX + 4);
-        const int gx = x0 + lx - 2, gy = y0 + ly - 2;
-        float v = 0.f;
-        if (gx >= 0 && gy >= 0 && gx < L.nx && gy < L.ny) {
-            const int i = gy * L.nx + gx;
-            if (L.dinv[i] != 0.f) v = x[i] + scale * yc[(gy >> SY) * cnx + (gx >> SX)];
-        }
-        s1[e] = v;
-    }
-    __syncthreads();
-    tile_sweep<kTX + 4, kTX + 2, 1>(L, om, b, x0, y0, s1, s2);
-    __syncthreads();
+    __shared__ TileMem T;
     double rz = 0.0, zq = 0.0;
-    for (int e = threadIdx.x; e < kTY * kTX; e += kT) {
-        const int ly = e / kTX, lx = e - ly * kTX;
-        const int gx = x0 + lx, gy = y0 + ly;
-        if (gx < L.nx && gy < L.ny) {
-            const int i = gy * L.nx + gx;
-            const float d = L.dinv[i];
-            float v = 0.f;
-            if (d != 0.f) {
-                const float c = s2[(ly + 1) * (kTX + 2) + lx + 1];
-                v = c + om * d * (b[i] - tile_apply<kTX + 2>(L, i, gx, gy, s2, ly + 1, lx + 1));
-            }
-            out[i] = v;
-            if (acc) {
-                rz += (double)b[i] * (double)v;
-                zq += (double)v * (double)q[i];
-            }
-        }
-    }
+    mg_up_tile<SX, SY>(L, om, scale, b, x, yc, cnx, out, acc ? q : nullptr, &rz, &zq, blockIdx.x * kTX,
+                       blockIdx.y * kTY, T);
     if (acc) {
         Acc *a = acc + ctl->slot;
         cta_add(rz, &a->rzn);
@@ -639,8 +689,9 @@ __device__ __forceinline__ float sm_apply(const SmLevel &L, int i, const float *
 }
 
 // dst = src + w D^-1 (b - A src) on the inside nodes, 0 outside.
+template <int NT>
 __device__ __forceinline__ void sm_sweep(const SmLevel &L, float om, const float *src, float *dst) {
-    for (int i = threadIdx.x; i < L.n; i += kBlockThreads) {
+    for (int i = threadIdx.x; i < L.n; i += NT) {
         const float d = L.dv[i];
         dst[i] = d != 0.f ? src[i] + om * d * (L.b[i] - sm_apply(L, i, src)) : 0.f;
     }
@@ -649,12 +700,9 @@ __device__ __forceinline__ void sm_sweep(const SmLevel &L, float om, const float
 // coef_smem: the levels' operator is copied to shared memory (7 floats per
 // node); otherwise it is read from its global arrays (3 floats per node in
 // shared memory: b, x, y), which lets larger levels into this kernel.
-__global__ void __launch_bounds__(kBlockThreads) k_mg_block(MgBlock P, const float *__restrict__ b_in,
-                                                            float *__restrict__ y_out, int coef_smem) {
-    pdl_wait();
-    pdl_launch();
-    extern __shared__ float sm[];
-    __shared__ SmLevel Ls[kMgMaxBlockLevels];
+template <int NT>
+__device__ __forceinline__ void mg_block_solve(const MgBlock &P, const float *b_in, float *y_out, int coef_smem, float *sm,
+                                               SmLevel *Ls) {
     if (threadIdx.x == 0) {
         float *p = sm;
         for (int l = 0; l < P.nb; ++l) {
@@ -684,7 +732,7 @@ __global__ void __launch_bounds__(kBlockThreads) k_mg_block(MgBlock P, const flo
     __syncthreads();
     for (int l = 0; l < P.nb; ++l) {
         const SmLevel &L = Ls[l];
-        for (int i = threadIdx.x; i < L.n; i += kBlockThreads) {
+        for (int i = threadIdx.x; i < L.n; i += NT) {
             if (coef_smem) {
                 L.ex[i] = P.ex[l][i];
                 L.ey[i] = P.ey[l][i];
@@ -701,11 +749,11 @@ __global__ void __launch_bounds__(kBlockThreads) k_mg_block(MgBlock P, const flo
     for (int l = 0; l + 1 < P.nb; ++l) {
         const SmLevel &L = Ls[l], &C = Ls[l + 1];
         const int sx = C.nx != L.nx, sy = C.ny != L.ny;
-        for (int i = threadIdx.x; i < L.n; i += kBlockThreads) L.y[i] = om * L.dv[i] * L.b[i];
+        for (int i = threadIdx.x; i < L.n; i += NT) L.y[i] = om * L.dv[i] * L.b[i];
         __syncthreads();
-        sm_sweep(L, om, L.y, L.x);
+        sm_sweep<NT>(L, om, L.y, L.x);
         __syncthreads();
-        for (int I = threadIdx.x; I < C.n; I += kBlockThreads) {
+        for (int I = threadIdx.x; I < C.n; I += NT) {
             const int R = I / C.nx, Cc = I - R * C.nx;
             float s = 0.f;
 #pragma unroll
@@ -723,7 +771,7 @@ __global__ void __launch_bounds__(kBlockThreads) k_mg_block(MgBlock P, const flo
     {  // bottom: y[idx[r]] = sum_c inv[r][c] b[idx[c]], one warp per row
         const SmLevel &B = Ls[P.nb - 1];
         const int lane = threadIdx.x & 31;
-        for (int r = threadIdx.x >> 5; r < P.m; r += kBlockThreads / 32) {
+        for (int r = threadIdx.x >> 5; r < P.m; r += NT / 32) {
             const float *row = P.inv + (size_t)r * P.m;
             float s = 0.f;
             for (int c = lane; c < P.m; c += 32) s = fmaf(row[c], B.b[P.idx[c]], s);
@@ -736,18 +784,27 @@ __global__ void __launch_bounds__(kBlockThreads) k_mg_block(MgBlock P, const flo
     for (int l = P.nb - 2; l >= 0; --l) {
         const SmLevel &L = Ls[l], &C = Ls[l + 1];
         const int sx = C.nx != L.nx, sy = C.ny != L.ny;
-        for (int i = threadIdx.x; i < L.n; i += kBlockThreads) {
+        for (int i = threadIdx.x; i < L.n; i += NT) {
             const int r = i / L.nx, c = i - r * L.nx;
             L.y[i] = L.dv[i] != 0.f ? L.x[i] + P.scale * C.y[(r >> sy) * C.nx + (c >> sx)] : 0.f;
         }
         __syncthreads();
-        sm_sweep(L, om, L.y, L.x);
+        sm_sweep<NT>(L, om, L.y, L.x);
         __syncthreads();
-        sm_sweep(L, om, L.x, L.y);
+        sm_sweep<NT>(L, om, L.x, L.y);
         __syncthreads();
     }
     const SmLevel &T = Ls[0];
-    for (int i = threadIdx.x; i < T.n; i += kBlockThreads) y_out[i] = T.y[i];
+    for (int i = threadIdx.x; i < T.n; i += NT) y_out[i] = T.y[i];
+}
+
+__global__ void __launch_bounds__(kBlockThreads) k_mg_block(MgBlock P, const float *__restrict__ b_in,
+                                                            float *__restrict__ y_out, int coef_smem) {
+    pdl_wait();
+    pdl_launch();
+    extern __shared__ float sm[];
+    __shared__ SmLevel Ls[kMgMaxBlockLevels];
+    mg_block_solve<kBlockThreads>(P, b_in, y_out, coef_smem, sm, Ls);
 }
 
 // ------------------------------------------------ one-cluster coarse levels
@@ -1173,13 +1230,37 @@ int launch_mg_cluster(const MgCluster &P, cudaStream_t s) {
     return OEC_OK;
 }
 
+// The coarse levels' plan from level B on for one CTA.
+MgBlock mg_block_plan(const oec_mg_t *mg, int B) {
+    MgBlock P{};
+    P.nb = mg->nlevels - B;
+    P.m = mg->ncoarse;
+    for (int k = B; k < mg->nlevels; ++k) {
+        const oec_mg_level_t &l = mg->levels[k];
+        const int j = k - B;
+        P.nx[j] = l.nx;
+        P.ny[j] = l.ny;
+        P.ex[j] = l.ex;
+        P.ey[j] = l.ey;
+        P.leak[j] = l.leak;
+        P.dinv[j] = l.dinv;
+    }
+    P.idx = mg->coarse_idx;
+    P.inv = mg->coarse_inv;
+    P.om = mg->omega;
+    P.scale = mg->scale;
+    return P;
+}
+
 // One V-cycle z = M r; with acc, also the flexible-CG dot products r.z and
 // z.q into acc[ctl->slot] (q the operator image of the current direction).
 // Levels above the coarse solve run as tiled kernels over the whole GPU; the
-// coarse levels run in one cluster (mg->cluster_top) or one CTA.
+// coarse levels run in one cluster (mg->cluster_top) or one CTA.  (The tiled
+// levels of at most 300,000 nodes and the one-CTA solve in one cooperative
+// launch, a grid barrier per level, lost to the overlapped launches: 1024^2
+// V-cycle 88 against 75 us, 128^2 39 against 31 us.)
 int mg_cycle(const oec_mg_t *mg, const float *r, float *z, const float *q, Acc *acc, const Ctl *ctl,
              cudaStream_t s) {
-    const int L = mg->nlevels;
     MgCluster C;
     const bool clustered = mg_cluster_plan(mg, C);
     const int B = clustered ? mg_cluster_top_level(mg) : mg->block_level;
@@ -1206,22 +1287,7 @@ int mg_cycle(const oec_mg_t *mg, const float *r, float *z, const float *q, Acc *
         }
         OEC_TRY(launch_mg_cluster(C, s));
     } else {
-        MgBlock P{};
-        P.nb = L - B;
-        P.m = mg->ncoarse;
-        for (int k = B; k < L; ++k) {
-            const int j = k - B;
-            P.nx[j] = lv[k].nx;
-            P.ny[j] = lv[k].ny;
-            P.ex[j] = lv[k].ex;
-            P.ey[j] = lv[k].ey;
-            P.leak[j] = lv[k].leak;
-            P.dinv[j] = lv[k].dinv;
-        }
-        P.idx = mg->coarse_idx;
-        P.inv = mg->coarse_inv;
-        P.om = mg->omega;
-        P.scale = mg->scale;
+        const MgBlock P = mg_block_plan(mg, B);
         const size_t smem = mg_block_smem(mg);
         if (smem > 48 * 1024) {
             // the largest dynamic shared-memory size enabled so far, per device
