@@ -18,8 +18,15 @@ def device():
     return _DEV
 
 
+# the handle alone: torch.cuda.current_stream builds a Stream object around it
+# (2.2 us a call against 0.1, paid by every launch of the package)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def stream():
     """Handle of the current torch CUDA stream, as the C ABI's void* stream."""
+    if _raw_stream is not None:
+        return _raw_stream(device().index)
     return torch.cuda.current_stream(device()).cuda_stream
 
 
