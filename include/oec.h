@@ -461,7 +461,7 @@ typedef struct oec_nd {
     int32_t n_levels;
     int32_t max_front;         /* inputs that a CTA's shared memory holds: at least 16 * OEC_ND_WARP_IN, a multiple of 4 */
     int32_t n_tiles;
-    int32_t pad;
+    int32_t ctas;              /* most CTAs of a solve with levels, when several run at a time (0: all that fit) */
     int64_t n_mat;
     oec_nd_level_t level[OEC_ND_MAX_LEVELS];
     const oec_nd_tile_t *tiles; /* [n_tiles], 16-byte aligned */

@@ -28,9 +28,28 @@ from .autotune import Autotuner
 from .buildup import Buildup
 from .grid import Grid
 from .lu_setup import factor
+from .nd_setup import CTAS
 from .poissonSolver import PoissonSolver
 
 GRID_KEYS = (("nx", 128), ("ny", 128), ("lx", 0.04), ("ly", 0.04), ("boundType", 1))
+
+
+# A direct solve on all SMs leaves no room beside it, and on small grids most of
+# its time is barriers and dependent loads: solves of several branches side by
+# side on a part of the SMs each take longer alone and less together.  Quarters
+# are the smallest useful part (batch step of 6 runs on 96-192^2 in 6 branches: 290 us
+# with whole solves, 248 halves, 221 quarters, 235 sixths).  A grid above the
+# average gets more, as the other branches may end up waiting for it (16 runs on
+# 256-1024^2: 2.70 -> 2.38 ms in 4 branches, 2.70 -> 2.20 in 16; 64 runs in 16
+# 11.97 -> 9.10).
+SOLVE_PARTS = 4
+
+
+def solve_ctas(nodes, mean_nodes, branches):
+    """CTAs for one direct solve on a grid of `nodes` nodes beside those of the
+    other branches, whose grids have `mean_nodes` on average (0: no limit)."""
+    parts = min(SOLVE_PARTS, branches, max(1, round(branches * mean_nodes / nodes)))
+    return CTAS // parts if parts > 1 else 0
 
 
 class BatchedBuildup:
@@ -93,6 +112,9 @@ class BatchedBuildup:
         return tuple(b._step_signature() for b in self.runs)
 
     def _capture(self, nb):
+        nodes = [b.ps.n_nodes for b in self.runs]
+        for _, ps in self.shared.values():
+            ps.shareSolve(solve_ctas(ps.n_nodes, sum(nodes) / len(nodes), nb))
         for b in self.runs:
             b.ps.prepare()
         while len(self._streams) < nb:

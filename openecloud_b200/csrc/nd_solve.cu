@@ -15,7 +15,7 @@
 // barriers and the dependent loads around them small ones.  Measured (warm,
 // per solve) against the level-scheduled factors with their dense tail:
 // 33 x 25 rectangle 6.2 against 270 us, 128^2 circle 20.5 against 146 us, 512^2
-// ellipse 115 against 1400 us, 1024^2 ellipse 320 us against 9.1 ms; the blocks
+// ellipse 111 against 1400 us, 1024^2 ellipse 312 us against 9.1 ms; the blocks
 // take 4, 44, 264 and 1049 MB (the 1024^2 tail inverses alone took 4.3 GB).
 // Tried and dropped: only 128-thread CTAs, eight to an SM (45 us at 128^2: every
 // CTA gathers a long front's inputs anew); fetching the next pass's first blocks
@@ -169,11 +169,21 @@ __device__ __forceinline__ void run_tiles(const NdArgs &a, const oec_nd_tile_t *
     const int slots = L < 32 ? kWarps : parts, slot = L < 32 ? tid >> 5 : part;
     vec += group * (a.nd.max_front / kGroups);
     red += group * 2 * GT;
-    const int step = gridDim.x * kGroups;
-    for (int k = blockIdx.x + group * gridDim.x; k < n_tiles; k += step) {
+    // with several tiles to a CTA: neighbouring ones, so that the front's inputs
+    // are gathered once (quarters, with short inputs, lost by the uneven tiles that
+    // lie together: 1024^2 312 -> 328 us)
+    const int gid = blockIdx.x + group * gridDim.x, groups = gridDim.x * kGroups;
+    int k = gid, end = n_tiles, step = groups, front = -1;
+    if (GT == kNdThreads && n_tiles > groups) {
+        k = (int)((int64_t)n_tiles * gid / groups);
+        end = (int)((int64_t)n_tiles * (gid + 1) / groups);
+        step = 1;
+    }
+    for (; k < end; k += step) {
         const oec_nd_tile_t t = load_tile(tiles + k);
-        if (tid == 0 && k + step < n_tiles) prefetch_l1(tiles + k + step);
-        gather<FWD>(a, t, children, tid, GT, vec);
+        if (tid == 0 && k + step < end) prefetch_l1(tiles + k + step);
+        if (GT != kNdThreads || t.piv0 != front) gather<FWD>(a, t, children, tid, GT, vec);
+        front = t.piv0;
         const int oa = t.o0 + tid;  // this thread's output
         const bool has = tid < width;
         const double base = has ? out_base<FWD>(a, t, oa, children) : 0.0;
@@ -274,7 +284,7 @@ int64_t pass_ctas(const oec_nd_pass_t &p) {
 
 int nd_solve(const oec_nd_t *nd, const double *q, double *phi, double *work, cudaStream_t s) {
     if (nd->n <= 0 || nd->n_levels < 1 || nd->n_levels > OEC_ND_MAX_LEVELS || nd->max_front < kNdWarps * kNdWarpVec ||
-        nd->max_front > OEC_ND_MAX_FRONT || nd->max_front % 4 || nd->n_bnd < 0 || nd->n_outside < 0 || !nd->tiles || !nd->piv_node ||
+        nd->max_front > OEC_ND_MAX_FRONT || nd->max_front % 4 || nd->n_bnd < 0 || nd->n_outside < 0 || nd->ctas < 0 || !nd->tiles || !nd->piv_node ||
         !nd->mat || (nd->n_levels > 1 && (!nd->piv_src || !nd->bnd_node || !nd->bnd_src)) ||
         (nd->n_outside > 0 && !nd->outside))
         return OEC_ERR_INVALID;
@@ -302,7 +312,9 @@ int nd_solve(const oec_nd_t *nd, const double *q, double *phi, double *work, cud
     // every CTA resident at once: the barrier between levels is the grid's
     int per_sm = 0;
     OEC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_nd_solve, kNdThreads, smem));
-    const int grid = (int)std::min<int64_t>(need, (int64_t)sm_count() * std::min(per_sm, kNdPerSm));
+    int64_t most = (int64_t)sm_count() * std::min(per_sm, kNdPerSm);
+    if (nd->ctas > 0) most = std::min<int64_t>(most, nd->ctas);
+    const int grid = (int)std::min(need, most);
     if (grid < 1) return OEC_ERR_CUDA;
     void *args[] = {&a};
     OEC_CUDA_TRY(cudaLaunchCooperativeKernel((void *)k_nd_solve, dim3(grid), dim3(kNdThreads), args, smem, s));

@@ -42,7 +42,7 @@ class Nd_t(ctypes.Structure):
     _P = ctypes.c_void_p
     _fields_ = [("n", ctypes.c_int32), ("n_nodes", ctypes.c_int32), ("n_bnd", ctypes.c_int32),
                 ("n_outside", ctypes.c_int32), ("n_levels", ctypes.c_int32), ("max_front", ctypes.c_int32),
-                ("n_tiles", ctypes.c_int32), ("pad", ctypes.c_int32), ("n_mat", ctypes.c_int64),
+                ("n_tiles", ctypes.c_int32), ("ctas", ctypes.c_int32), ("n_mat", ctypes.c_int64),
                 ("level", NdLevel_t * MAX_LEVELS), ("tiles", _P), ("piv_node", _P), ("piv_src", _P),
                 ("bnd_node", _P), ("bnd_src", _P), ("outside", _P), ("mat", _P)]
 

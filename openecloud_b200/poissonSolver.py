@@ -365,6 +365,12 @@ class PoissonSolver:
         s._mg = None if self._mg is None else PoissonSolver._mg_state(self._mg["shared"])
         return s
 
+    def shareSolve(self, ctas):
+        """At most `ctas` CTAs (0: all that fit) for each direct solve from now
+        on, of this solver and its siblings.  The results do not depend on it."""
+        if self._lu_t.nd:
+            self._nd_t.ctas = int(ctas)
+
     def applyOperator(self, x):
         """A x on the inside nodes (device f64 [npExt] in and out)."""
         y = torch.empty_like(x)

@@ -84,3 +84,29 @@ def test_fronts_on_the_device(gpu, p, levels, monkeypatch):
     ps.solve(q)
     assert np.array_equal(ps.getPhi(), x)
     assert np.all(np.delete(x, inside) == 0.0)
+
+
+def test_parts_of_the_device_for_the_solves_of_a_batch():
+    from openecloud_b200.batch import solve_ctas
+    assert solve_ctas(1000, 1000, 1) == 0
+    assert [solve_ctas(1000, 1000, b) for b in (2, 3, 4, 64)] == [148, 98, 74, 74]
+    assert solve_ctas(9000, 3000, 4) == 0 and solve_ctas(4000, 3000, 4) == 98 and solve_ctas(10, 3000, 4) == 74
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("p", [(64, 48, 0.04, 0.04, 1), (128, 128, 0.04, 0.04, 1), (402, 301, 0.09, 0.036, 1)])
+def test_solve_on_a_part_of_the_device(gpu, p):
+    """Fewer CTAs (several tiles to each, down to all of them to one) give the
+    bits of the whole device."""
+    from openecloud_b200.poissonSolver import PoissonSolver
+    g, a, inside, q, phi, tol = _case(p)
+    ps = PoissonSolver(g)
+    ps.solve(q)
+    x = ps.getPhi()
+    assert np.linalg.norm(x - phi) <= tol * np.linalg.norm(phi)
+    s = ps.sibling()
+    for ctas in (1, 7, 74, 148, 295, 10000, 0):
+        ps.shareSolve(ctas)
+        s.phi.fill_(-1.0)
+        s.solve(q)
+        assert np.array_equal(s.getPhi(), x), ctas
