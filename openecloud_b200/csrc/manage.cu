@@ -28,9 +28,9 @@
 namespace oec {
 namespace {
 
-constexpr int kSortThreads = 256;                      // threads per sort CTA (8 warps)
+constexpr int kSortThreads = 512;                      // threads per sort CTA (16 warps)
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kPerLane = 16;                            // keys per thread
+constexpr int kPerLane = 8;                             // keys per thread (16 with 256 threads: 231 -> 217 us)
 constexpr int kTile = kSortThreads * kPerLane;          // keys per sort tile (one CTA): 4096
 constexpr int kWarpKeys = 32 * kPerLane;                // a warp's consecutive keys in the tile
 
@@ -67,7 +67,7 @@ __device__ __forceinline__ int blk_scan(int v, int *tot, int *sh) {
 // digit-major, hist[d * ntiles + tile].
 __global__ void __launch_bounds__(kSortThreads) k_digit_hist(const uint32_t *__restrict__ keys, const int32_t *n_p,
                                                              int shift, int ntiles, int *__restrict__ hist) {
-    __shared__ int h[kSortWarps][256];
+    __shared__ int h[kSortWarps][256];  // 16 KB
     const int n = *n_p;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int d = threadIdx.x; d < kSortWarps * 256; d += kSortThreads) (&h[0][0])[d] = 0;
@@ -104,29 +104,43 @@ __global__ void __launch_bounds__(kDigitScanT) k_digit_scan(int *__restrict__ hi
     if (threadIdx.x == 0) total[blockIdx.x] = carry;
 }
 
+// The lanes of the warp that hold a key (`mine`) with this lane's digit, by a vote
+// per bit.  __match_any_sync takes a step per distinct value, some 30 of them in
+// a round of random digits (sort of 2.2e6 by weight with 16 keys a thread 244 -> 231 us).
+__device__ __forceinline__ unsigned warp_peers(unsigned mine, int d) {
+    unsigned peers = mine;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool bit = (d >> b) & 1;
+        const unsigned set = __ballot_sync(kFullMask, bit);
+        peers &= bit ? set : ~set;
+    }
+    return peers;
+}
+
 // Stable scatter of one tile (kTile keys) by the digit at `shift`.  Warp w
-// owns the tile's keys w*512 .. w*512+511 and walks them in 16 rounds of 32
+// owns the tile's keys w*256 .. w*256+255 and walks them in 8 rounds of 32
 // consecutive keys (coalesced loads); a key's place among the equal digits
 // of its warp is the warp's running count of that digit (shared memory, one
 // counter row per warp) plus the lanes below it in the round with the same
-// digit (a warp match).  After the rounds the counts of the lower warps give
+// digit (warp_peers).  After the rounds the counts of the lower warps give
 // each warp's start inside the tile's run of a digit, and the scanned tile
 // histogram the run's start in the output, so the order is (digit, tile,
 // warp, round, lane) = stable.  The tile is put in that order in shared memory
 // first and written from there, so that a digit's keys leave in one run: written
 // from the registers every key was a sector of its own (2.2e6 pairs per pass
 // 38 -> 27 us).
-__global__ void __launch_bounds__(kSortThreads) k_scatter(const uint32_t *__restrict__ keys,
+__global__ void __launch_bounds__(kSortThreads, 3) k_scatter(const uint32_t *__restrict__ keys,
                                                           const int32_t *__restrict__ vals, const int32_t *n_p,
                                                           int shift, int ntiles, const int *__restrict__ offs,
                                                           const int *__restrict__ total,
                                                           uint32_t *__restrict__ okeys, int32_t *__restrict__ ovals) {
-    static_assert(kSortThreads == 256, "a thread per digit");
+    static_assert(kSortThreads >= 256 && kTile < 1 << 16, "a thread per digit, 16-bit counts");
     __shared__ uint32_t sk[kTile];
     __shared__ int32_t sv[kTile];
     __shared__ int first[256];  // output place of a digit's first key minus its place in the tile
     __shared__ int sh[32];
-    __shared__ int cnt[kSortWarps][256];  // running digit counts, then each warp's start in a digit's run
+    __shared__ uint16_t cnt[kSortWarps][256];  // running digit counts, then each warp's start in a digit's run
     const int n = *n_p;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
@@ -146,12 +160,12 @@ __global__ void __launch_bounds__(kSortThreads) k_scatter(const uint32_t *__rest
 #pragma unroll
     for (int r = 0; r < kPerLane; ++r) {
         const bool valid = base + r * 32 < n;
-        const int d = valid ? (int)((k[r] >> shift) & 255u) : 256;
-        const unsigned peers = __match_any_sync(kFullMask, d);
+        const int d = (int)((k[r] >> shift) & 255u);
+        const unsigned peers = warp_peers(__ballot_sync(kFullMask, valid), d);
         int rank = 0;
         if (valid) rank = cnt[w][d] + __popc(peers & below);
         __syncwarp();
-        if (valid && (peers & below) == 0) cnt[w][d] += __popc(peers);
+        if (valid && (peers & below) == 0) cnt[w][d] = (uint16_t)(rank + __popc(peers));
         __syncwarp();
         dr[r] = valid ? (d << 16 | rank) : -1;
     }
@@ -159,18 +173,23 @@ __global__ void __launch_bounds__(kSortThreads) k_scatter(const uint32_t *__rest
     // digit d's run in the tile: its start, and in it each warp's start (the
     // counts of the lower warps)
     const int d0 = threadIdx.x;
+    const bool digit = d0 < 256;
     int run = 0;
+    if (digit) {
 #pragma unroll
-    for (int q = 0; q < kSortWarps; ++q) run += cnt[q][d0];
-    const int out0 = blk_scan(total[d0], nullptr, sh) + offs[d0 * ntiles + blockIdx.x];
+        for (int q = 0; q < kSortWarps; ++q) run += cnt[q][d0];
+    }
+    const int out0 = blk_scan(digit ? total[d0] : 0, nullptr, sh);
     int nk;
     int at = blk_scan(run, &nk, sh);
-    first[d0] = out0 - at;
+    if (digit) {
+        first[d0] = out0 + offs[d0 * ntiles + blockIdx.x] - at;
 #pragma unroll
-    for (int q = 0; q < kSortWarps; ++q) {
-        const int c = cnt[q][d0];
-        cnt[q][d0] = at;
-        at += c;
+        for (int q = 0; q < kSortWarps; ++q) {
+            const int c = cnt[q][d0];
+            cnt[q][d0] = (uint16_t)at;
+            at += c;
+        }
     }
     __syncthreads();
 #pragma unroll
@@ -231,12 +250,14 @@ __global__ void k_permute(oec_particles_t p, const int32_t *__restrict__ perm, o
 // The same through rows of 32 bytes: a particle in random order is then one
 // sector instead of seven (2.2e6 particles by weight 94 -> 60 us with the
 // packing).  An order close to the stored one is faster field by field.
+__device__ __forceinline__ void pack_row(const oec_particles_t &p, int i, float4 *__restrict__ rows) {
+    rows[2 * (int64_t)i] = make_float4(__int_as_float(p.cell[i]), p.ox[i], p.oy[i], p.vx[i]);
+    rows[2 * (int64_t)i + 1] = make_float4(p.vy[i], p.vz[i], p.w[i], 0.f);
+}
+
 __global__ void k_pack_rows(oec_particles_t p, float4 *__restrict__ rows) {
     const int n = *p.count;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        rows[2 * (int64_t)i] = make_float4(__int_as_float(p.cell[i]), p.ox[i], p.oy[i], p.vx[i]);
-        rows[2 * (int64_t)i + 1] = make_float4(p.vy[i], p.vz[i], p.w[i], 0.f);
-    }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) pack_row(p, i, rows);
 }
 
 __global__ void k_permute_rows(const float4 *__restrict__ rows, const int32_t *__restrict__ perm, const int32_t *count,
@@ -257,14 +278,14 @@ __global__ void k_permute_rows(const float4 *__restrict__ rows, const int32_t *_
 }
 
 // ------------------------------------------------------- weight search
-// _searchSorted (particleManagement.pyx:244-262) on the weight-sorted store,
-// one thread per threshold, the reference's loop as written (it answers 0 as
-// soon as a[0] >= value): the first index with a[i] > value.
+// _searchSorted (particleManagement.pyx:244-262) on the weight-sorted store:
+// 0 when w[0] >= value, else the first index with w[i] > value.  A warp per
+// threshold takes 32 probes a round, five rounds of dependent loads for 2^24
+// weights where the reference's bisection has 24.
 __global__ void k_search_sorted2(const float *__restrict__ w, const int32_t *count, double lo, double hi,
                                  int32_t *out) {
-    const int t = threadIdx.x;
-    if (t > 1) return;
-    const double value = t == 0 ? lo : hi;
+    const int lane = threadIdx.x & 31;
+    const double value = threadIdx.x < 32 ? lo : hi;
     const int n = *count;
     int r;
     if (n <= 0) {
@@ -274,17 +295,19 @@ __global__ void k_search_sorted2(const float *__restrict__ w, const int32_t *cou
     } else if ((double)w[0] >= value) {
         r = 0;
     } else {
-        int i0 = 0, i2 = n - 1, i1 = (int)((i2 + i0) * 0.5);
-        while (i1 != i0) {
-            if ((double)w[i1] > value)
-                i2 = i1;
-            else
-                i0 = i1;
-            i1 = (int)((i2 + i0) * 0.5);
+        // w[i0] <= value < w[i2]
+        int i0 = 0, i2 = n - 1;
+        while (i2 - i0 > 1) {
+            const int step = (i2 - i0 + 32) / 33, i = min(i0 + (lane + 1) * step, i2);
+            const unsigned above = __ballot_sync(kFullMask, (double)w[i] > value);
+            const int below = above ? __ffs(above) - 1 : 32;  // probes before the first one above
+            const int a = i0;
+            if (below < 32) i2 = min(a + (below + 1) * step, i2);
+            i0 = min(a + below * step, i2 - 1);
         }
-        r = i1 + 1;
+        r = i0 + 1;
     }
-    out[t] = r;
+    if (lane == 0) out[threadIdx.x >> 5] = r;
 }
 
 // -------------------------------------------------------------- roulette
@@ -343,8 +366,9 @@ __global__ void k_clone_rows(oec_particles_t p, int n, int k, uint2 key, uint32_
 
 // ------------------------------------------------------------ local merge
 
-// Stats over particles [0, n): sum w, sum |v|^2 w^2 (f64, atomics).
+// Stats over particles [0, n): sum w, sum |v|^2 w^2 (f64, one atomic per sum and CTA).
 __global__ void k_wstats(oec_particles_t p, double *acc) {
+    __shared__ double sh[2][32];
     int n = *p.count;
     double sw = 0, sv = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -357,8 +381,14 @@ __global__ void k_wstats(oec_particles_t p, double *acc) {
         sv += __shfl_xor_sync(kFullMask, sv, o);
     }
     if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&acc[0], sw);
-        atomicAdd(&acc[1], sv);
+        sh[0][threadIdx.x >> 5] = sw;
+        sh[1][threadIdx.x >> 5] = sv;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        double t = 0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sh[threadIdx.x][w];
+        atomicAdd(&acc[threadIdx.x], t);
     }
 }
 
@@ -366,7 +396,9 @@ struct MergeArgs {
     oec_particles_t p;         // weight-sorted store
     int n_cand;                // merge candidates: the lightest n_cand particles
     int n_merge_target;        // merges wanted
-    const int32_t *order;      // candidates ordered by (cell, velocity key)
+    const int32_t *order;      // candidates in Morton order
+    const float4 *rows;        // candidates packed as k_pack_rows does, in store order
+    uint32_t *qual;            // a bit per pair: it passes the test
     double lam2;               // (ds / v_typical)^2 * lambda_factor^2
     double limit;              // factorDisLimit * ds (compared with the squared distance, as the reference)
     double dx, dy;
@@ -380,24 +412,38 @@ struct MergeArgs {
 };
 
 // Pair (2k, 2k+1) of the ordered candidates: qualifies when the weighted
-// phase-space distance passes the reference's test.
+// phase-space distance passes the reference's test.  The two lie anywhere in the
+// store, so they are read from packed rows, one sector each where the arrays
+// would take six, and the outcome is kept for k_pair_merge.  Bound by these
+// sectors.
 __global__ void k_pair_count(MergeArgs a) {
-    int npairs = a.n_cand / 2;
+    const int npairs = a.n_cand / 2, lane = threadIdx.x & 31;
     int q = 0;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < npairs; k += gridDim.x * blockDim.x) {
-        int i = a.order[2 * k], j = a.order[2 * k + 1];
-        int ix, iy, jx, jy;
-        split_cell(a.p.cell[i], a.nx, a.inv_nx, ix, iy);
-        split_cell(a.p.cell[j], a.nx, a.inv_nx, jx, jy);
-        double ddx = ((double)(ix - jx) + ((double)a.p.ox[i] - a.p.ox[j])) * a.dx;
-        double ddy = ((double)(iy - jy) + ((double)a.p.oy[i] - a.p.oy[j])) * a.dy;
-        double dvx = (double)a.p.vx[i] - a.p.vx[j], dvy = (double)a.p.vy[i] - a.p.vy[j],
-               dvz = (double)a.p.vz[i] - a.p.vz[j];
-        double d2 = ddx * ddx + ddy * ddy + a.lam2 * (dvx * dvx + dvy * dvy + dvz * dvz);
-        if (d2 < a.limit) ++q;
+    for (int k0 = blockIdx.x * blockDim.x + threadIdx.x - lane; k0 < npairs; k0 += gridDim.x * blockDim.x) {
+        const int k = k0 + lane;
+        bool near = false;
+        if (k < npairs) {
+            const int i = __ldg(a.order + 2 * k), j = __ldg(a.order + 2 * k + 1);
+            const float4 *ri = a.rows + 2 * (int64_t)i, *rj = a.rows + 2 * (int64_t)j;
+            const float4 pi = __ldg(ri), pj = __ldg(rj);
+            const float2 vi = __ldg(reinterpret_cast<const float2 *>(ri + 1));
+            const float2 vj = __ldg(reinterpret_cast<const float2 *>(rj + 1));
+            int ix, iy, jx, jy;
+            split_cell(__float_as_int(pi.x), a.nx, a.inv_nx, ix, iy);
+            split_cell(__float_as_int(pj.x), a.nx, a.inv_nx, jx, jy);
+            const double ddx = ((double)(ix - jx) + ((double)pi.y - pj.y)) * a.dx;
+            const double ddy = ((double)(iy - jy) + ((double)pi.z - pj.z)) * a.dy;
+            const double dvx = (double)pi.w - pj.w, dvy = (double)vi.x - vj.x, dvz = (double)vi.y - vj.y;
+            const double d2 = ddx * ddx + ddy * ddy + a.lam2 * (dvx * dvx + dvy * dvy + dvz * dvz);
+            near = d2 < a.limit;
+        }
+        const unsigned m = __ballot_sync(kFullMask, near);
+        if (lane == 0) {
+            a.qual[k0 >> 5] = m;
+            q += __popc(m);
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(kFullMask, q, o);
-    if ((threadIdx.x & 31) == 0 && q) atomicAdd(&a.counters[0], q);
+    if (lane == 0 && q) atomicAdd(&a.counters[0], q);
 }
 
 __global__ void k_pair_merge(MergeArgs a) {
@@ -406,19 +452,11 @@ __global__ void k_pair_merge(MergeArgs a) {
     double paccept = qual > 0 ? fmin(1.0, (double)a.n_merge_target / (double)qual) : 0.0;
     int done = 0;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < npairs; k += gridDim.x * blockDim.x) {
-        int i = a.order[2 * k], j = a.order[2 * k + 1];
-        int ix, iy, jx, jy;
-        split_cell(a.p.cell[i], a.nx, a.inv_nx, ix, iy);
-        split_cell(a.p.cell[j], a.nx, a.inv_nx, jx, jy);
-        double ddx = ((double)(ix - jx) + ((double)a.p.ox[i] - a.p.ox[j])) * a.dx;
-        double ddy = ((double)(iy - jy) + ((double)a.p.oy[i] - a.p.oy[j])) * a.dy;
-        double dvx = (double)a.p.vx[i] - a.p.vx[j], dvy = (double)a.p.vy[i] - a.p.vy[j],
-               dvz = (double)a.p.vz[i] - a.p.vz[j];
-        double d2 = ddx * ddx + ddy * ddy + a.lam2 * (dvx * dvx + dvy * dvy + dvz * dvz);
-        if (!(d2 < a.limit)) continue;
+        if (!(a.qual[k >> 5] >> (k & 31) & 1u)) continue;
         uint4 r = sf::philox4x32_10(make_uint4((uint32_t)k, a.call, 0u, 0x3e59u), a.key);
         double u0 = r.x * (1.0 / 4294967296.0), u1 = r.y * (1.0 / 4294967296.0);
         if (u0 >= paccept) continue;
+        const int i = a.order[2 * k], j = a.order[2 * k + 1];
         double wi = a.p.w[i], wj = a.p.w[j];
         int keep = (u1 < wi / (wi + wj)) ? i : j;  // keep with probability proportional to weight
         int drop = keep == i ? j : i;
@@ -440,6 +478,14 @@ __global__ void k_pair_merge(MergeArgs a) {
     }
     for (int o = 16; o > 0; o >>= 1) done += __shfl_xor_sync(kFullMask, done, o);
     if ((threadIdx.x & 31) == 0 && done) atomicAdd(&a.counters[1], done);
+}
+
+// The candidates' count, the empty bounding box and the zeroed counters.
+__global__ void k_merge_begin(int n_cand, int32_t *ncand, uint32_t *bbox, int32_t *counters) {
+    const int t = threadIdx.x;
+    if (t == 0) *ncand = n_cand;
+    if (t < 10) bbox[t] = t < 5 ? 0xffffffffu : 0u;
+    if (t < 2) counters[t] = 0;
 }
 
 // Weighted phase-space coordinates of the merge metric (localRandom :166-171):
@@ -503,9 +549,10 @@ __device__ __forceinline__ float key_float(uint32_t k) {
 
 // Candidate keys: 5-D Morton order (6 bits per axis, one common scale for all
 // axes so that the order follows the isotropic weighted metric): neighbours in
-// key order are close in (x, y, lambda v).
+// key order are close in (x, y, lambda v).  The candidates also go into packed
+// rows for k_pair_count.
 __global__ void k_cand_keys(oec_particles_t p, int n_cand, int nx, float inv_nx, double dx, double dy, double lam,
-                            const uint32_t *bbox, uint32_t *keys, int32_t *vals) {
+                            const uint32_t *bbox, uint32_t *keys, int32_t *vals, float4 *rows) {
     float lo[5], span = 0.f;
     for (int d = 0; d < 5; ++d) {
         lo[d] = key_float(bbox[d]);
@@ -522,6 +569,7 @@ __global__ void k_cand_keys(oec_particles_t p, int n_cand, int nx, float inv_nx,
             for (int d = 0; d < 5; ++d) key = (key << 1) | ((q[d] >> b) & 1u);
         keys[i] = key;
         vals[i] = i;
+        pack_row(p, i, rows);
     }
 }
 
@@ -560,6 +608,12 @@ extern "C" int64_t oec_sort_work_bytes(int64_t capacity) {
 
 // The digit totals, behind the histogram and its 256-byte slack.
 static int *digit_totals(int *hist, int64_t ntiles) { return hist + 256 * ntiles + 64; }
+
+// The packed rows, behind the digit totals.
+static float4 *packed_rows(int *hist, int64_t cap) {
+    const uintptr_t end = reinterpret_cast<uintptr_t>(digit_totals(hist, (cap + kTile - 1) / kTile) + 256);
+    return reinterpret_cast<float4 *>((end + 31) & ~uintptr_t(31));
+}
 
 // Stable radix sort of (keys, vals) pairs, keys in work; `bits` significant key bits.
 static int radix_sort(uint32_t *keys, int32_t *vals, uint32_t *k2, int32_t *v2, int *hist, const int32_t *n_dev,
@@ -609,8 +663,7 @@ extern "C" int oec_sort_particles(oec_particles_t *p, oec_particles_t *tmp, int3
     if (column == 6) {
         k_permute<<<g, 256, 0, s>>>(*p, vout, *tmp);
     } else {
-        const uintptr_t end = reinterpret_cast<uintptr_t>(digit_totals(hist, (cap + kTile - 1) / kTile) + 256);
-        float4 *rows = reinterpret_cast<float4 *>((end + 31) & ~uintptr_t(31));
+        float4 *rows = packed_rows(hist, cap);
         k_pack_rows<<<g, 256, 0, s>>>(*p, rows);
         k_permute_rows<<<g, 256, 0, s>>>(rows, vout, p->count, *tmp);
     }
@@ -621,7 +674,7 @@ extern "C" int oec_sort_particles(oec_particles_t *p, oec_particles_t *tmp, int3
 extern "C" int oec_weight_thresholds(const oec_particles_t *p, double lo, double hi, int32_t *out_dev,
                                      void *stream) {
     if (!vp2(p) || !out_dev) return OEC_ERR_INVALID;
-    k_search_sorted2<<<1, 32, 0, as_stream(stream)>>>(p->w, p->count, lo, hi, out_dev);
+    k_search_sorted2<<<1, 64, 0, as_stream(stream)>>>(p->w, p->count, lo, hi, out_dev);
     OEC_LAUNCH_CHECK();
     return OEC_OK;
 }
@@ -702,13 +755,12 @@ extern "C" int oec_cell_merge(const oec_grid_t *grid, oec_particles_t *p, int32_
     int *hist = reinterpret_cast<int *>(v2 + cap);
     int32_t *ncand_dev = reinterpret_cast<int32_t *>(hist + 256 * ((cap + kTile - 1) / kTile));
     uint32_t *bbox = reinterpret_cast<uint32_t *>(ncand_dev + 1);  // 10 words (inside the 256-byte slack)
-    uint32_t init[10] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u, 0u, 0u};
-    OEC_CUDA_TRY(cudaMemcpyAsync(ncand_dev, &n_cand, sizeof(int32_t), cudaMemcpyHostToDevice, s));
-    OEC_CUDA_TRY(cudaMemcpyAsync(bbox, init, sizeof(init), cudaMemcpyHostToDevice, s));
-    OEC_CUDA_TRY(cudaMemsetAsync(counters_dev, 0, 2 * sizeof(int32_t), s));
+    float4 *rows = packed_rows(hist, cap);
+    k_merge_begin<<<1, 32, 0, s>>>(n_cand, ncand_dev, bbox, counters_dev);
     int g = persistent_grid((n_cand + 255) / 256 + 1, 8);
-    k_cand_bbox<<<persistent_grid((n_cand + 255) / 256 + 1, 2), 256, 0, s>>>(*p, n_cand, gc.nx, 1.0f / (float)gc.nx, gc.dx, gc.dy, lambda, bbox);
-    k_cand_keys<<<g, 256, 0, s>>>(*p, n_cand, gc.nx, 1.0f / (float)gc.nx, gc.dx, gc.dy, lambda, bbox, keys, vals);
+    k_cand_bbox<<<g, 256, 0, s>>>(*p, n_cand, gc.nx, 1.0f / (float)gc.nx, gc.dx, gc.dy, lambda, bbox);
+    k_cand_keys<<<g, 256, 0, s>>>(*p, n_cand, gc.nx, 1.0f / (float)gc.nx, gc.dx, gc.dy, lambda, bbox, keys, vals,
+                                rows);
     uint32_t *kout;
     int32_t *vout;
     int rc = radix_sort(keys, vals, k2, v2, hist, ncand_dev, cap, 32, s, &kout, &vout);
@@ -718,6 +770,8 @@ extern "C" int oec_cell_merge(const oec_grid_t *grid, oec_particles_t *p, int32_
     a.n_cand = n_cand;
     a.n_merge_target = n_merge;
     a.order = vout;
+    a.rows = rows;
+    a.qual = kout == keys ? k2 : keys;  // the sort's other key buffer
     a.lam2 = lambda * lambda;
     a.limit = limit;
     a.dx = gc.dx;
@@ -732,6 +786,5 @@ extern "C" int oec_cell_merge(const oec_grid_t *grid, oec_particles_t *p, int32_
     k_pair_count<<<g, 256, 0, s>>>(a);
     k_pair_merge<<<g, 256, 0, s>>>(a);
     OEC_LAUNCH_CHECK();
-    OEC_CUDA_TRY(cudaStreamSynchronize(s));  // n_cand lives on this stack frame
     return OEC_OK;
 }
