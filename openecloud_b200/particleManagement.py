@@ -73,7 +73,11 @@ def localRandom(gridObj, particlesObj, particleBoundaryObj, targetMacroParticleC
     n = P.getMacroParticleCount()
     target = int(targetMacroParticleCount)
     s = D.stream()
-    meanWeight = P.getMeanWeight()
+    # both sums at once, before the sort (they do not depend on the order)
+    acc = D.zeros(2, torch.float64)
+    _lib.call("oec_weight_stats", P.c_particles(), acc.data_ptr(), s)
+    sum_w, sum_v2w2 = (float(x) for x in D.to_numpy(acc))
+    meanWeight = sum_w / n
     goal = meanWeight * n / target
     maxT, minT = thresholdFactor * goal, goal / thresholdFactor
     ds = min(gridObj.getDx(), gridObj.getDy())
@@ -96,9 +100,7 @@ def localRandom(gridObj, particlesObj, particleBoundaryObj, targetMacroParticleC
     if 2 * to_merge + to_split >= n:
         f = 0.95 * n / (2 * to_merge + to_split)
         to_merge, to_split = int(to_merge * f), int(to_split * f)
-    acc = D.zeros(2, torch.float64)
-    _lib.call("oec_weight_stats", P.c_particles(), acc.data_ptr(), s)
-    vt = float(np.sqrt(acc[1].item())) / (n * meanWeight)
+    vt = float(np.sqrt(sum_v2w2)) / (n * meanWeight)
     vt = max(vt, 1.e-12 * c)
     rows = D.empty((max(to_split, 1), 6), torch.float64)
     _lib.call("oec_split_rows", gridObj.c_grid(), P.c_particles(), n, to_split, rows.data_ptr(), s)
