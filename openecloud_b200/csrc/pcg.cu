@@ -369,6 +369,36 @@ __global__ void __launch_bounds__(kT) k_direction32(int G, const float *__restri
     if (more) cudaGraphSetConditional(h_inner, 1);
 }
 
+// End of an iteration that began with the V-cycle (one thread): k_direction32's
+// check, and the sums of the next iteration cleared.
+__device__ __forceinline__ void check_step(Acc *a, Ctl *c, int it, double pqs, int max_iter, oec_pcg_stats_t *stats,
+                                           cudaGraphConditionalHandle h_inner) {
+    const double rrs = *(volatile double *)&a->rr;
+    const int it1 = it + 1, total = c->total + 1;
+    c->it = it1;
+    c->total = total;
+    stats->iterations = total;
+    bool more = total < max_iter;
+    if (!isfinite(rrs)) {
+        stats->breakdown = 1;
+        more = false;
+    } else {
+        const double rel_in = sqrt(rrs);
+        if (rel_in <= c->inner_tol) {
+            more = false;
+        } else if (rel_in < 0.9 * c->best) {
+            c->best = rel_in;
+            c->best_at = it1;
+        } else if (it1 - c->best_at >= 1024) {
+            more = false;
+        }
+    }
+    // the next V-cycle accumulates its dot products from zero
+    c->pq_prev = pqs;
+    a->pq = a->rr = a->rzn = a->zq = 0.0;
+    if (more) cudaGraphSetConditional(h_inner, 1);
+}
+
 // The inner iteration's CG part when the preconditioner runs first in the
 // loop body (the multigrid V-cycle: z = M r with acc.rzn += r.z and
 // acc.zq += z.q of the previous direction's q): the new direction
@@ -423,34 +453,98 @@ __global__ void __launch_bounds__(kT) k_cg_step(int nx, int G, const float *__re
     }
     grid.sync();
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    const double rrs = a->rr;
-    const int it1 = it + 1, total = c->total + 1;
-    c->it = it1;
-    c->total = total;
-    stats->iterations = total;
-    bool more = total < max_iter;
-    if (!isfinite(rrs)) {
-        stats->breakdown = 1;
-        more = false;
-    } else {
-        const double rel_in = sqrt(rrs);
-        if (rel_in <= c->inner_tol) {
-            more = false;
-        } else if (rel_in < 0.9 * c->best) {
-            c->best = rel_in;
-            c->best_at = it1;
-        } else if (it1 - c->best_at >= 1024) {
-            more = false;
-        }
-    }
-    // the next V-cycle accumulates its dot products from zero
-    c->pq_prev = pqs;
-    a->pq = a->rr = a->rzn = a->zq = 0.0;
-    if (more) cudaGraphSetConditional(h_inner, 1);
+    check_step(a, c, it, pqs, max_iter, stats, h_inner);
 }
 
-// Start of the inner loop of k_cg_step: d = 0, q = 0, arms the loop (r was
-// scaled by k_scale32).
+// The same part of the iteration on grids too large for grid-wide barriers, as
+// two launches.  First: p = z + beta p_old at a node and its four neighbours
+// (formed anew for each, so the direction takes no pass of its own; the two
+// directions alternate between two vectors, by the parity of the iteration),
+// q = A p, acc.pq += p.q.  It disarms the loop.
+__global__ void __launch_bounds__(kT) k_dir_apply32(int nx, int G, const float *__restrict__ ex,
+                                                    const float *__restrict__ ey, const uint8_t *__restrict__ in,
+                                                    const float *__restrict__ z, float *p0, float *p1,
+                                                    float *__restrict__ q, Acc *acc, const Ctl *c,
+                                                    cudaGraphConditionalHandle h_inner) {
+    pdl_wait();
+    pdl_launch();
+    Acc *a = acc + c->slot;
+    const int it = c->it;
+    if (blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(h_inner, 0);
+    float beta = 0.f;
+    if (it > 0) {
+        const double b = -a->zq / c->pq_prev;
+        beta = isfinite(b) ? (float)b : 0.f;
+    }
+    float *pn = it & 1 ? p1 : p0;
+    const float *po = it & 1 ? p0 : p1;
+    const auto at = [&](int j) { return it > 0 ? fmaf(beta, po[j], z[j]) : z[j]; };
+    double pq = 0.0;
+    for (int i = blockIdx.x * kT + threadIdx.x; i < G; i += gridDim.x * kT) {
+        const float pi = at(i);
+        float v = 0.0f;
+        if (in[i]) {
+            v = ex[i] * (pi - at(i + 1)) + ex[i - 1] * (pi - at(i - 1)) + ey[i] * (pi - at(i + nx)) +
+                ey[i - nx] * (pi - at(i - nx));
+            pq += (double)pi * (double)v;
+        }
+        pn[i] = pi;
+        q[i] = v;
+    }
+    cta_add(pq, &a->pq);
+}
+
+// Second: the step into d and r with |r|^2, and in the last CTA to finish the
+// convergence check of k_direction32.  The check stands before the next V-cycle,
+// so a converged residual is not preconditioned once more.
+__global__ void __launch_bounds__(kT) k_step_check32(int G, const float *p0, const float *p1,
+                                                     const float *__restrict__ q, float *__restrict__ d,
+                                                     float *__restrict__ r, Acc *acc, Ctl *c, int max_iter,
+                                                     oec_pcg_stats_t *stats, cudaGraphConditionalHandle h_inner) {
+    pdl_wait();
+    pdl_launch();
+    Acc *a = acc + c->slot;
+    const int it = c->it;
+    const float *p = it & 1 ? p1 : p0;
+    const double pq = a->pq, rz = a->rzn;
+    if (pq > 0.0 && isfinite(rz)) {
+        const float alpha = (float)(rz / pq);
+        double rr = 0.0;
+        const int n4 = aligned16(p, q) && aligned16(d, r) ? G >> 2 : 0;
+        for (int k = blockIdx.x * kT + threadIdx.x; k < n4; k += gridDim.x * kT) {
+            const float4 pv = reinterpret_cast<const float4 *>(p)[k], qv = reinterpret_cast<const float4 *>(q)[k];
+            float4 dv = reinterpret_cast<float4 *>(d)[k], rv = reinterpret_cast<float4 *>(r)[k];
+            dv = make_float4(fmaf(alpha, pv.x, dv.x), fmaf(alpha, pv.y, dv.y), fmaf(alpha, pv.z, dv.z),
+                             fmaf(alpha, pv.w, dv.w));
+            rv = make_float4(fmaf(-alpha, qv.x, rv.x), fmaf(-alpha, qv.y, rv.y), fmaf(-alpha, qv.z, rv.z),
+                             fmaf(-alpha, qv.w, rv.w));
+            reinterpret_cast<float4 *>(d)[k] = dv;
+            reinterpret_cast<float4 *>(r)[k] = rv;
+            rr += (double)rv.x * (double)rv.x;
+            rr += (double)rv.y * (double)rv.y;
+            rr += (double)rv.z * (double)rv.z;
+            rr += (double)rv.w * (double)rv.w;
+        }
+        for (int i = 4 * n4 + blockIdx.x * kT + threadIdx.x; i < G; i += gridDim.x * kT) {
+            d[i] = fmaf(alpha, p[i], d[i]);
+            const float ri = fmaf(-alpha, q[i], r[i]);
+            r[i] = ri;
+            rr += (double)ri * (double)ri;
+        }
+        cta_add(rr, &a->rr);
+    } else if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a->rr = __longlong_as_double(0x7ff8000000000000LL);  // nobody adds to it
+    }
+    if (threadIdx.x != 0) return;  // thread 0 made the CTA's add
+    __threadfence();
+    if (atomicAdd(&c->ticket, 1) != (int)gridDim.x - 1) return;
+    __threadfence();
+    c->ticket = 0;
+    check_step(a, c, it, pq, max_iter, stats, h_inner);
+}
+
+// Start of the inner loop that begins with the V-cycle: d = 0, q = 0, arms the
+// loop (r was scaled by k_scale32).
 __global__ void __launch_bounds__(kT) k_init_cg(int G, float *__restrict__ d, float *__restrict__ q,
                                                 cudaGraphConditionalHandle h_inner) {
     for (int i = blockIdx.x * kT + threadIdx.x; i < G; i += gridDim.x * kT) {
@@ -1378,7 +1472,11 @@ bool valid_stencil(const oec_stencil_t *st) {
 //       [k_scale32, M r] k_init32        (arms h_inner)
 //       WHILE inner:                     (h_inner: disarmed by k_apply32,
 //         k_apply32, k_update32,          re-armed by k_direction32's check)
-//         [M r (+ dots)], k_direction32
+//         [M r, dots], k_direction32
+//     or with the multigrid
+//       k_scale32, k_init_cg
+//       WHILE inner:                     (disarmed and re-armed by the CG step)
+//         V-cycle with dots, k_cg_step or k_dir_apply32 and k_step_check32
 //       k_accumulate64
 //   [k_fallback_flag, IF fallback: LU solve]
 // Every loop ends: each refinement raises the refinement count (at most
@@ -1523,8 +1621,10 @@ int build_solve(const SolveArgs &a, cudaStream_t s) {
             BodyCapture c2;
             OEC_TRY(c2.begin(1, b_work));
             OEC_CUDA_TRY(cudaGraphConditionalHandleCreate(&h_inner, b_work, 0, 0));
-            if (coop_grid > 0) {
-                // multigrid: V-cycle first in the loop body, then the CG step
+            if (pc == OEC_PRECOND_MG) {
+                // multigrid: V-cycle first in the loop body, then the CG step (one
+                // cooperative launch or two: cg_step_grid).  Against apply, update,
+                // V-cycle and direction: cold 1024^2 solve 2354 -> 2089 us, same iterations.
                 k_scale32<<<grid, kT, 0, c2.s>>>(G, w.r64, w.ctl, w.r);
                 k_init_cg<<<grid, kT, 0, c2.s>>>(G, w.d, w.q, h_inner);
                 OEC_LAUNCH_CHECK();
@@ -1532,12 +1632,20 @@ int build_solve(const SolveArgs &a, cudaStream_t s) {
                 BodyCapture c3;
                 OEC_TRY(c3.begin(2, b_inner));
                 OEC_TRY(external_apply(pc, a.ctx, w.r, w.z, w.q, w.acc, w.ctl, c3.s));
+                if (coop_grid == 0) {
+                    OEC_CUDA_TRY(launch_overlapped(k_dir_apply32, dim3(grid), dim3(kT), 0, c3.s, nx, G, st->ex32,
+                                                   st->ey32, st->inside, w.z, w.p, w.zn, w.q, w.acc, w.ctl, h_inner));
+                    OEC_CUDA_TRY(launch_overlapped(k_step_check32, dim3(grid), dim3(kT), 0, c3.s, G, w.p, w.zn, w.q,
+                                                   w.d, w.r, w.acc, w.ctl, a.max_iter, a.stats, h_inner));
+                }
                 int max_iter = a.max_iter;
                 void *args[] = {(void *)&nx, (void *)&G, (void *)&st->ex32, (void *)&st->ey32, (void *)&st->inside,
                                 (void *)&w.z, (void *)&w.p, (void *)&w.q, (void *)&w.d, (void *)&w.r,
                                 (void *)&w.acc, (void *)&w.ctl, (void *)&max_iter, (void *)&a.stats,
                                 (void *)&h_inner};
-                OEC_CUDA_TRY(cudaLaunchCooperativeKernel((void *)k_cg_step, dim3(coop_grid), dim3(kT), args, 0, c3.s));
+                if (coop_grid > 0)
+                    OEC_CUDA_TRY(
+                        cudaLaunchCooperativeKernel((void *)k_cg_step, dim3(coop_grid), dim3(kT), args, 0, c3.s));
                 OEC_TRY(c3.end());
             } else {
                 if (external) {
@@ -1557,9 +1665,7 @@ int build_solve(const SolveArgs &a, cudaStream_t s) {
                     OEC_CUDA_TRY(launch_overlapped(k_update32, dim3(grid), dim3(kT), 0, c3.s, G, st->dinv32, pc, w.p, w.q,
                                                    w.d, w.r, w.z, w.acc, w.ctl));
                     OEC_LAUNCH_CHECK();
-                    if (pc == OEC_PRECOND_MG) {
-                        OEC_TRY(external_apply(pc, a.ctx, w.r, w.z, w.q, w.acc, w.ctl, c3.s));
-                    } else if (external) {
+                    if (external) {
                         OEC_TRY(external_apply(pc, a.ctx, w.r, w.zn, nullptr, nullptr, nullptr, c3.s));
                         OEC_CUDA_TRY(launch_overlapped(k_zdots32, dim3(grid), dim3(kT), 0, c3.s, G, w.r, w.zn, w.q, w.z,
                                                        w.acc, w.ctl));

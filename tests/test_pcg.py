@@ -189,6 +189,35 @@ def test_pcg_matches_lu_and_reference(gpu, name, precond):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("p", [(361, 359, 0.04, 0.04, 1), (362, 361, 0.04, 0.04, 1), (517, 299, 0.09, 0.036, 0)])
+@pytest.mark.parametrize("limit", [20000, 4])
+def test_mg_pcg_on_both_sides_of_the_cooperative_step(gpu, p, limit):
+    """131,043 nodes take the cooperative step, 132,132 and more the two kernels
+    (an odd count too, so the last nodes go one by one); cold, then from the last
+    solution, then out of iterations with the direct solve behind."""
+    from openecloud_b200.grid import Grid
+    from openecloud_b200.poissonSolver import PoissonSolver
+    g = Grid(*p)
+    ps = PoissonSolver(g, method="pcg", precond="mg", pcgTol=1e-8, pcgMaxIter=limit)
+    ins = ps.insidePointsInd
+    q = np.zeros(ps.n_nodes)
+    q[ins] = np.random.default_rng(p[0]).normal(size=ins.size) * 1e-12 + 1e-12
+    lu = PoissonSolver(g)
+    for scale in (1.0, 1.001):
+        ps.solve(scale * q)
+        st = ps.lastStats
+        lu.solve(scale * q)
+        if limit == 4:
+            assert st.converged == 0 and ps.nFallbacks >= 1 and rel_err(ps.getPhi(), lu.getPhi()) <= 1e-12
+            return
+        assert st.converged == 1 and st.rel_residual <= 1e-8 and ps.nFallbacks == 0
+        assert 0 < st.iterations <= 60
+        res = ps.systemMatrix.dot(ps.getPhi()[ins]) - scale * q[ins]
+        assert np.linalg.norm(res) <= 1.5e-8 * np.linalg.norm(scale * q[ins])
+        assert rel_err(ps.getPhi(), lu.getPhi()) <= 1e-6
+
+
+@pytest.mark.gpu
 def test_pcg_warm_start_and_fallback(gpu):
     import torch
     from openecloud_b200 import device as D
