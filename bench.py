@@ -354,7 +354,7 @@ def gpu_passage():
     b = Buildup(seed=1000, n_steps_table=2501)
     s_lu = b.run(2500)
     nfin = int(b.history()[0][-1])
-    out = {"workload": PASSAGE, "s_per_passage": s_lu, "solver": "LU (f64, level-scheduled + dense tail)",
+    out = {"workload": PASSAGE, "s_per_passage": s_lu, "solver": "direct (f64, nested-dissection fronts)",
            "final_macro_particles": nfin}
     m = Buildup(seed=1000, n_steps_table=2501)
     m.ps.method, m.ps.precond = "pcg", "mg"

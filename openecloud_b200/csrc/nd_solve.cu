@@ -19,7 +19,9 @@
 // take 4, 44, 264 and 1049 MB (the 1024^2 tail inverses alone took 4.3 GB).
 // Tried and dropped: only 128-thread CTAs, eight to an SM (45 us at 128^2: every
 // CTA gathers a long front's inputs anew); fetching the next pass's first blocks
-// into L1 or L2 ahead of the barrier (1024^2 330 -> 344 us).
+// into L1 or L2 ahead of the barrier (1024^2 330 -> 344 us); fetching a warp's or a
+// group's next block into L2 behind the current one (with E, 1024^2 330 -> 328 us, but
+// 512^2 119 -> 121 and 1000 x 700 274 -> 277 us).
 #include <stdint.h>
 
 #include <cooperative_groups.h>
