@@ -126,7 +126,7 @@ struct Ctl {
     double inv_rnorm;          // 1 / ||r|| of the current refinement
     double coef;               // scale32 * ||r||: weight of the f32 correction
     double best;               // best inner residual so far (stagnation window)
-    double pq_prev;            // p.Ap of the previous inner iteration (k_cg_step)
+    double pq_prev;            // p.Ap of the previous inner iteration (k_dir_apply32)
     int slot, it, total, refine, best_at, ticket;
     oec_pcg_stats_t stats;     // stats of the synchronous entry point
 };
@@ -401,66 +401,14 @@ __device__ __forceinline__ void check_step(Acc *a, Ctl *c, int it, double pqs, i
 
 // The inner iteration's CG part when the preconditioner runs first in the
 // loop body (the multigrid V-cycle: z = M r with acc.rzn += r.z and
-// acc.zq += z.q of the previous direction's q): the new direction
-// p = z + beta p (beta = -(z.q)/(p.q), flexible CG; p = z in the first
-// iteration), q = A p with p.q, the step alpha = (r.z)/(p.q) into d and r
-// with |r|^2, and the convergence check of k_direction32 -- one cooperative
-// launch with grid-wide barriers between the parts instead of three launches
-// (all CTAs resident).  A non-positive or non-finite curvature leaves d and r
-// unchanged and ends the loop as a breakdown.
-__global__ void __launch_bounds__(kT) k_cg_step(int nx, int G, const float *__restrict__ ex,
-                                                const float *__restrict__ ey, const uint8_t *__restrict__ in,
-                                                const float *__restrict__ z, float *__restrict__ p,
-                                                float *__restrict__ q, float *__restrict__ d, float *__restrict__ r,
-                                                Acc *acc, Ctl *c, int max_iter, oec_pcg_stats_t *stats,
-                                                cudaGraphConditionalHandle h_inner) {
-    cooperative_groups::grid_group grid = cooperative_groups::this_grid();
-    Acc *a = acc + c->slot;
-    const int it = c->it;
-    if (blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(h_inner, 0);
-    float beta = 0.f;
-    if (it > 0) {
-        double b = -a->zq / c->pq_prev;
-        beta = isfinite(b) ? (float)b : 0.f;
-    }
-    const int stride = gridDim.x * kT;
-    for (int i = blockIdx.x * kT + threadIdx.x; i < G; i += stride) p[i] = it > 0 ? fmaf(beta, p[i], z[i]) : z[i];
-    grid.sync();
-    double pq = 0.0;
-    for (int i = blockIdx.x * kT + threadIdx.x; i < G; i += stride) {
-        float v = 0.0f;
-        if (in[i]) {
-            v = apply_at(i, nx, ex, ey, p);
-            pq += (double)p[i] * (double)v;
-        }
-        q[i] = v;
-    }
-    cta_add(pq, &a->pq);
-    grid.sync();
-    const double pqs = a->pq, rz = a->rzn;
-    double rr = 0.0;
-    if (pqs > 0.0 && isfinite(rz)) {
-        const float alpha = (float)(rz / pqs);
-        for (int i = blockIdx.x * kT + threadIdx.x; i < G; i += stride) {
-            d[i] = fmaf(alpha, p[i], d[i]);
-            const float ri = fmaf(-alpha, q[i], r[i]);
-            r[i] = ri;
-            rr += (double)ri * (double)ri;
-        }
-        cta_add(rr, &a->rr);
-    } else if (blockIdx.x == 0 && threadIdx.x == 0) {
-        a->rr = __longlong_as_double(0x7ff8000000000000LL);
-    }
-    grid.sync();
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    check_step(a, c, it, pqs, max_iter, stats, h_inner);
-}
-
-// The same part of the iteration on grids too large for grid-wide barriers, as
-// two launches.  First: p = z + beta p_old at a node and its four neighbours
-// (formed anew for each, so the direction takes no pass of its own; the two
-// directions alternate between two vectors, by the parity of the iteration),
-// q = A p, acc.pq += p.q.  It disarms the loop.
+// acc.zq += z.q of the previous direction's q), as two launches.  First:
+// p = z + beta p_old (beta = -(z.q)/(p.q), flexible CG; p = z in the first
+// iteration) at a node and its four neighbours -- formed anew for each, so the
+// direction takes no pass of its own; the directions alternate between two
+// vectors, by the parity of the iteration -- q = A p, acc.pq += p.q.  It disarms the
+// loop.  (One cooperative launch with grid barriers between the parts loses at
+// every size: cold solves 40 x 30 442 against 421 us, 128^2 622 against 604, 256^2 890
+// against 845, 360 x 355 1112 against 986.)
 __global__ void __launch_bounds__(kT) k_dir_apply32(int nx, int G, const float *__restrict__ ex,
                                                     const float *__restrict__ ey, const uint8_t *__restrict__ in,
                                                     const float *__restrict__ z, float *p0, float *p1,
@@ -494,8 +442,9 @@ __global__ void __launch_bounds__(kT) k_dir_apply32(int nx, int G, const float *
     cta_add(pq, &a->pq);
 }
 
-// Second: the step into d and r with |r|^2, and in the last CTA to finish the
-// convergence check of k_direction32.  The check stands before the next V-cycle,
+// Second: the step alpha = (r.z)/(p.q) into d and r with |r|^2, and in the last CTA
+// to finish the convergence check of k_direction32.  A non-positive or non-finite
+// curvature leaves d and r unchanged and ends the loop as a breakdown.  The check stands before the next V-cycle,
 // so a converged residual is not preconditioned once more.
 __global__ void __launch_bounds__(kT) k_step_check32(int G, const float *p0, const float *p1,
                                                      const float *__restrict__ q, float *__restrict__ d,
@@ -1476,7 +1425,7 @@ bool valid_stencil(const oec_stencil_t *st) {
 //     or with the multigrid
 //       k_scale32, k_init_cg
 //       WHILE inner:                     (disarmed and re-armed by the CG step)
-//         V-cycle with dots, k_cg_step or k_dir_apply32 and k_step_check32
+//         V-cycle with dots, k_dir_apply32, k_step_check32
 //       k_accumulate64
 //   [k_fallback_flag, IF fallback: LU solve]
 // Every loop ends: each refinement raises the refinement count (at most
@@ -1564,42 +1513,12 @@ int capture_graph(cudaStream_t s, cudaGraph_t *g) {
 }
 
 // Records the whole solve into the capture of s.
-// Grids up to this many nodes take the cooperative k_cg_step: its grid
-// barriers cost less than three launches only while the passes are short
-// (measured cold solves, 15 / 23 iterations: 128^2 circle 0.826 -> 0.778 ms,
-// 1024^2 ellipse 2.83 -> 3.24 ms).
-constexpr int kCgStepMaxNodes = 1 << 17;
-
-// Grid of the cooperative k_cg_step for G nodes on this device: at most two
-// resident CTAs per SM, so that the whole grid fits beside other work (0:
-// a grid above kCgStepMaxNodes, cooperative launches unavailable, or
-// OEC_CG_STEP=0 in the environment; the iteration then runs as three
-// kernels).
-int cg_step_grid(int G) {
-    if (G > kCgStepMaxNodes) return 0;
-    static std::atomic<int> cached[kMaxDevices];
-    const int per_sm = per_device_cached(cached, [] {
-        const char *e = getenv("OEC_CG_STEP");
-        if (e && e[0] == '0') return 0;
-        int dev = 0, coop = 0, b = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cg_step, kT, 0) != cudaSuccess)
-            b = 0;
-        cudaGetLastError();
-        return b < 2 ? b : 2;
-    });
-    if (per_sm <= 0) return 0;
-    return persistent_grid((G + kT - 1) / kT, per_sm);
-}
-
 int build_solve(const SolveArgs &a, cudaStream_t s) {
     const oec_stencil_t *st = a.st;
     const int nx = st->nx, G = st->nx * st->ny;
     const int grid = persistent_grid((G + kT - 1) / kT, 4);
     const int pc = a.precond;
     const bool external = pc == OEC_PRECOND_CNN || pc == OEC_PRECOND_MG;
-    const int coop_grid = pc == OEC_PRECOND_MG ? cg_step_grid(G) : 0;
     Work w = carve(a.work, G);
     OEC_CUDA_TRY(cudaMemsetAsync(w.ctl, 0, sizeof(Ctl), s));
     OEC_CUDA_TRY(cudaMemsetAsync(a.stats, 0, sizeof(oec_pcg_stats_t), s));
@@ -1622,9 +1541,9 @@ int build_solve(const SolveArgs &a, cudaStream_t s) {
             OEC_TRY(c2.begin(1, b_work));
             OEC_CUDA_TRY(cudaGraphConditionalHandleCreate(&h_inner, b_work, 0, 0));
             if (pc == OEC_PRECOND_MG) {
-                // multigrid: V-cycle first in the loop body, then the CG step (one
-                // cooperative launch or two: cg_step_grid).  Against apply, update,
-                // V-cycle and direction: cold 1024^2 solve 2354 -> 2089 us, same iterations.
+                // multigrid: V-cycle first in the loop body, then the CG step.  Against
+                // apply, update, V-cycle and direction: cold 1024^2 solve 2354 -> 2089 us,
+                // same iterations.
                 k_scale32<<<grid, kT, 0, c2.s>>>(G, w.r64, w.ctl, w.r);
                 k_init_cg<<<grid, kT, 0, c2.s>>>(G, w.d, w.q, h_inner);
                 OEC_LAUNCH_CHECK();
@@ -1632,20 +1551,10 @@ int build_solve(const SolveArgs &a, cudaStream_t s) {
                 BodyCapture c3;
                 OEC_TRY(c3.begin(2, b_inner));
                 OEC_TRY(external_apply(pc, a.ctx, w.r, w.z, w.q, w.acc, w.ctl, c3.s));
-                if (coop_grid == 0) {
-                    OEC_CUDA_TRY(launch_overlapped(k_dir_apply32, dim3(grid), dim3(kT), 0, c3.s, nx, G, st->ex32,
-                                                   st->ey32, st->inside, w.z, w.p, w.zn, w.q, w.acc, w.ctl, h_inner));
-                    OEC_CUDA_TRY(launch_overlapped(k_step_check32, dim3(grid), dim3(kT), 0, c3.s, G, w.p, w.zn, w.q,
-                                                   w.d, w.r, w.acc, w.ctl, a.max_iter, a.stats, h_inner));
-                }
-                int max_iter = a.max_iter;
-                void *args[] = {(void *)&nx, (void *)&G, (void *)&st->ex32, (void *)&st->ey32, (void *)&st->inside,
-                                (void *)&w.z, (void *)&w.p, (void *)&w.q, (void *)&w.d, (void *)&w.r,
-                                (void *)&w.acc, (void *)&w.ctl, (void *)&max_iter, (void *)&a.stats,
-                                (void *)&h_inner};
-                if (coop_grid > 0)
-                    OEC_CUDA_TRY(
-                        cudaLaunchCooperativeKernel((void *)k_cg_step, dim3(coop_grid), dim3(kT), args, 0, c3.s));
+                OEC_CUDA_TRY(launch_overlapped(k_dir_apply32, dim3(grid), dim3(kT), 0, c3.s, nx, G, st->ex32, st->ey32,
+                                               st->inside, w.z, w.p, w.zn, w.q, w.acc, w.ctl, h_inner));
+                OEC_CUDA_TRY(launch_overlapped(k_step_check32, dim3(grid), dim3(kT), 0, c3.s, G, w.p, w.zn, w.q, w.d,
+                                               w.r, w.acc, w.ctl, a.max_iter, a.stats, h_inner));
                 OEC_TRY(c3.end());
             } else {
                 if (external) {

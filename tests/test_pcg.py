@@ -191,10 +191,10 @@ def test_pcg_matches_lu_and_reference(gpu, name, precond):
 @pytest.mark.gpu
 @pytest.mark.parametrize("p", [(361, 359, 0.04, 0.04, 1), (362, 361, 0.04, 0.04, 1), (517, 299, 0.09, 0.036, 0)])
 @pytest.mark.parametrize("limit", [20000, 4])
-def test_mg_pcg_on_both_sides_of_the_cooperative_step(gpu, p, limit):
-    """131,043 nodes take the cooperative step, 132,132 and more the two kernels
-    (an odd count too, so the last nodes go one by one); cold, then from the last
-    solution, then out of iterations with the direct solve behind."""
+def test_mg_pcg_grid_sizes(gpu, p, limit):
+    """Node counts that four divides and others (whose last nodes go one by one);
+    cold, then from the last solution, then out of iterations with the direct
+    solve behind."""
     from openecloud_b200.grid import Grid
     from openecloud_b200.poissonSolver import PoissonSolver
     g = Grid(*p)
