@@ -662,8 +662,9 @@ __global__ void k_push_begin(int32_t *n_absorbed, unsigned long long *__restrict
 // samples instead of four 3 % of the CTAs of a 512-row grid passed by chance
 // and held up the rest (2^24 electrons: 362 against 335 us).
 __device__ __forceinline__ bool chunk_is_local(const FusedArgs &a, int n) {
-    const int base = min((int)blockIdx.x * kChunk, n - 1), span = min(kChunk, n - base);
-    if (span <= 0) return true;
+    const int base = (int)blockIdx.x * kChunk;
+    if (base >= n) return true;  // no chunk for this CTA: an empty store has no cell to read
+    const int span = min(kChunk, n - base);
     const int c0 = a.cell[base], c1 = a.cell[base + span / 3], c2 = a.cell[base + 2 * span / 3],
               c3 = a.cell[base + span - 1];
     const int lo = min(min(c0, c1), min(c2, c3)), hi = max(max(c0, c1), max(c2, c3));

@@ -45,3 +45,31 @@ def test_random_and_cell_order_agree(gpu, n, bound, btype):
     assert np.array_equal(a[order], b) and np.array_equal(ina[order], inb)
     # the deposit is exact: every survivor's whole quantised charge is on the grid
     assert fa.sum() == np.rint(rows[ina == 1, 5].astype(np.float32).astype(np.float64) * sa).sum()
+
+
+@pytest.mark.parametrize("bound,btype", [(0, 0), (1, 1), (1, 2)])
+def test_empty_store(gpu, bound, btype):
+    """A store without particles (every one was removed): nothing is read, absorbed or
+    deposited, and what lies in the arrays stays as it was."""
+    import torch
+    from openecloud_b200.grid import Grid
+    from openecloud_b200.particleBoundary import AbsorbElliptical, AbsorbRectangular
+    from openecloud_b200.particles import Particles
+    g = Grid(40, 30, 0.04, 0.06, bound)
+    P = Particles("electrons", "variableWeight")
+    P.setParticleData(np.tile([0.001, 0.002, 1e5, 2e5, 3e5, 1.0], (2000, 1)))
+    P._bind(g)
+    P.setMacroParticleCount(0)
+    P._deposit_buffers(g)
+    P._rho_fix.fill_(7)
+    P._status.fill_(0)
+    before = {k: v.clone() for k, v in P.soa().items()}
+    e = P.fieldTable(g, np.ones(2 * g.getNpExt()), 2)
+    b = P.fieldTable(g, np.ones(3 * g.getNpExt()), 3) if btype == 2 else None
+    bd = (AbsorbRectangular if bound == 0 else AbsorbElliptical)(g, P)
+    for _ in range(2):
+        P.pushGatherDeposit(g, e, 3e-11, btype, bd, bCellTable=b)
+    torch.cuda.synchronize()
+    assert P.getMacroParticleCount() == 0 and not P._rho_fix.any()
+    assert all(torch.equal(P.soa()[k], before[k]) for k in before)
+    assert not any(P.status().values())
