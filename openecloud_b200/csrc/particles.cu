@@ -697,7 +697,9 @@ __global__ void __launch_bounds__(kThreads, fused_min_blocks(TB, KIND)) k_push_g
     NodeWindow nw{win, 0, 0};
     if (DEP)
         for (int e = threadIdx.x; e < 2 * kWinWords; e += kThreads) win[e] = 0u;
-    const bool local = !DEP || chunk_is_local(a, n);
+    // One answer for the CTA: a warp that sampled after others had begun to write moved cells
+    // would take the other loop alone.  The barrier also ends the clearing of the windows.
+    const bool local = !DEP || !__syncthreads_or(!chunk_is_local(a, n));
     pdl_wait();
     if (!local) {
         for (int chunk = blockIdx.x; chunk < nchunks; chunk += gridDim.x) {

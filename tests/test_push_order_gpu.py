@@ -73,3 +73,42 @@ def test_empty_store(gpu, bound, btype):
     assert P.getMacroParticleCount() == 0 and not P._rho_fix.any()
     assert all(torch.equal(P.soa()[k], before[k]) for k in before)
     assert not any(P.status().values())
+
+
+@pytest.mark.parametrize("rows_apart", [7, 8, 9])
+def test_chunks_at_the_limit_of_the_deposit_choice(gpu, rows_apart):
+    """Chunks whose first and last particle lie 8 rows apart, the limit up to which a CTA
+    takes the windows, and whose particles cross many rows in the push, so that a choice
+    made again from moved cells would come out differently: every launch deposits what
+    the same particles deposit in random order."""
+    import torch
+    from openecloud_b200.grid import Grid
+    from openecloud_b200.particleBoundary import AbsorbRectangular
+    from openecloud_b200.particles import Particles
+    g = Grid(64, 96, 0.04, 0.06, 0)
+    dx, dy, n = g.getDx(), g.getDy(), 40 * 1024
+    rng = np.random.default_rng(rows_apart)
+    k, chunk = np.arange(n) % 1024, np.arange(n) // 1024
+    cell_y = 30 + chunk % 20 + np.rint(k * rows_apart / 1023.0)
+    rows = np.empty((n, 6))
+    rows[:, 0] = (20 + rng.integers(0, 3, n) + rng.uniform(0.1, 0.9, n)) * dx - 0.02
+    rows[:, 1] = (cell_y + rng.uniform(0.1, 0.9, n)) * dy - 0.03
+    rows[:, 2], rows[:, 4] = rng.normal(0, 1e6, n), 0.0
+    rows[:, 3] = rng.uniform(-12, 12, n) * dy / 3e-11
+    rows[:, 5] = rng.uniform(0.5, 2.0, n)
+    e = np.zeros(2 * g.getNpExt())
+
+    def step(r):
+        P = Particles("electrons", "variableWeight")
+        P.setBConst([0.0, 0.1, 0.0])
+        P._bind(g)
+        out = []
+        for _ in range(30):
+            P.setParticleData(r)
+            P.pushGatherDeposit(g, P.fieldTable(g, e, 2), 3e-11, 1, AbsorbRectangular(g, P))
+            out.append(P._rho_fix.clone())
+        torch.cuda.synchronize()
+        return out
+
+    got, want = step(rows), step(rows[rng.permutation(n)])
+    assert want[0].any() and all(torch.equal(x, want[0]) for x in got + want)
