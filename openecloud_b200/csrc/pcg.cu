@@ -481,9 +481,11 @@ __global__ void __launch_bounds__(kT) k_step_check32(int G, const float *p0, con
             rr += (double)ri * (double)ri;
         }
         cta_add(rr, &a->rr);
-    } else if (blockIdx.x == 0 && threadIdx.x == 0) {
-        a->rr = __longlong_as_double(0x7ff8000000000000LL);  // nobody adds to it
+    } else {
+        if (blockIdx.x == 0 && threadIdx.x == 0) a->rr = __longlong_as_double(0x7ff8000000000000LL);  // nobody adds to it
+        __syncthreads();
     }
+    // the CTA has read the sums (a barrier on either way), so the last CTA may clear them
     if (threadIdx.x != 0) return;  // thread 0 made the CTA's add
     __threadfence();
     if (atomicAdd(&c->ticket, 1) != (int)gridDim.x - 1) return;

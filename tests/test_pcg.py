@@ -414,3 +414,37 @@ def test_mg_vcycle_large_block_matches_tiled(gpu, top, cluster_top):
     got = D.to_numpy(zd).astype(np.float64)
     want = vcycle(host, r.astype(np.float64), omega=mg["c"].omega, scale=mg["c"].scale, dinv=dinv)
     assert np.max(np.abs(got - want)) <= 2e-4 * np.max(np.abs(want))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("p", [(40, 24, 0.04, 0.03, 1), (512, 512, 0.09, 0.036, 1)])
+def test_mg_breakdown_leaves_the_iterate_and_falls_back(gpu, p):
+    """A preconditioner that gives NaN: the first step's curvature is not finite, so the inner
+    loop ends as a breakdown after one iteration, the iterate keeps its bits (seen without
+    the fallback), and with it the direct solve answers."""
+    import ctypes
+    import torch
+    from openecloud_b200 import device as D
+    from openecloud_b200.grid import Grid
+    from openecloud_b200.poissonSolver import PRECOND, PcgStats_t, PoissonSolver, _declare
+    ps = PoissonSolver(Grid(*p), method="pcg", precond="mg", warmStart="previous")
+    ps.prepare()
+    ps._mg["shared"]["cinv"].fill_(float("nan"))
+    rng = np.random.default_rng(3)
+    q, start = np.zeros(ps.n_nodes), np.zeros(ps.n_nodes)
+    q[ps.insidePointsInd] = rng.normal(size=ps.insidePointsInd.size) * 1e-9
+    start[ps.insidePointsInd] = rng.normal(size=ps.insidePointsInd.size)
+    qd = torch.as_tensor(q, device="cuda")
+    ps.solveDevice(qd, method="lu")
+    want = ps.getPhi()
+    ctx = ctypes.cast(ctypes.pointer(ps._mg["c"]), ctypes.c_void_p)
+    for k in range(20):
+        phi, st = torch.as_tensor(start, device="cuda"), PcgStats_t()
+        _declare().oec_pcg_solve(ctypes.byref(ps._stencil), qd.data_ptr(), phi.data_ptr(), ps.pcgTol, ps.pcgMaxIter,
+                                 PRECOND["mg"], ctx, ps._pcg_work.data_ptr(), ctypes.byref(st), D.stream())
+        assert (st.breakdown, st.iterations, st.converged) == (1, 1, 0)
+        assert np.array_equal(phi.cpu().numpy(), start)
+        ps.phi.zero_()
+        ps.solveDevice(qd)
+        assert ps.lastStats.breakdown == 1 and ps.nFallbacks == k + 1
+        assert np.array_equal(ps.getPhi(), want)
