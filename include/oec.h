@@ -526,8 +526,8 @@ typedef struct oec_lu {
 #define OEC_LU_HEAD_ONE_CTA 3      /* one CTA per factor, the vector in shared memory */
 
 /* phi = A^-1 q on the inside nodes, 0 elsewhere (poissonSolver.pyx:85).
- * q_dev, phi_dev: [n_nodes]; work_dev: n + (n - head) doubles, or with nd
- * n + nd->n_bnd. */
+ * q_dev, phi_dev: [n_nodes], and they may overlap; work_dev: n + (n - head)
+ * doubles, or with nd n + nd->n_bnd. */
 int oec_lu_solve(const oec_lu_t *lu, const double *q_dev, double *phi_dev, double *work_dev, void *stream);
 
 /* y = A x, CSR with int32 indices (E = phiToE . phi, poissonSolver.pyx:87). */

@@ -42,6 +42,7 @@ struct NdArgs {
     oec_nd_t nd;
     const double *q;
     double *phi, *y, *u;
+    bool staged;  // q shares memory with phi: the root's part of q lies in y (k_nd_stage)
 };
 
 __device__ __forceinline__ double2 load_mat(const double *p) { return __ldg(reinterpret_cast<const double2 *>(p)); }
@@ -105,15 +106,16 @@ __device__ __forceinline__ double2 partial(const double *__restrict__ M, int ld,
 // The inputs of a tile into v: forward the pivots' right-hand side with the
 // children's updates, backward phi on the boundary.
 template <bool FWD>
-__device__ __forceinline__ void gather(const NdArgs &a, const oec_nd_tile_t &t, bool children, int first, int step,
-                                       double *v) {
+__device__ __forceinline__ void gather(const NdArgs &a, const oec_nd_tile_t &t, bool children, bool root, int first,
+                                       int step, double *v) {
+    const bool staged = FWD && root && a.staged;
     const int4 *src = reinterpret_cast<const int4 *>(a.nd.piv_src) + t.piv0;
     const int32_t *node = FWD ? a.nd.piv_node + t.piv0 : a.nd.bnd_node + t.bnd0;
 #pragma unroll 2
     for (int i = first; i < t.n_in; i += step) {
         const int k = __ldg(node + i);
         if (FWD) {
-            double x = __ldg(a.q + k);
+            double x = staged ? __ldcg(a.y + t.piv0 + i) : __ldg(a.q + k);
             if (children) x += child_sum(__ldg(src + i), a.u);
             v[i] = x;
         } else {
@@ -184,7 +186,7 @@ __device__ __forceinline__ void run_tiles(const NdArgs &a, const oec_nd_tile_t *
     for (; k < end; k += step) {
         const oec_nd_tile_t t = load_tile(tiles + k);
         if (tid == 0 && k + step < end) prefetch_l1(tiles + k + step);
-        if (GT != kNdThreads || t.piv0 != front) gather<FWD>(a, t, children, tid, GT, vec);
+        if (GT != kNdThreads || t.piv0 != front) gather<FWD>(a, t, children, root, tid, GT, vec);
         front = t.piv0;
         const int oa = t.o0 + tid;  // this thread's output
         const bool has = tid < width;
@@ -218,7 +220,7 @@ __device__ __forceinline__ void run_fronts(const NdArgs &a, const oec_nd_tile_t 
         const oec_nd_tile_t t = load_tile(tiles + k);
         if (k + step < n_tiles) prefetch_l1(tiles + k + step);
         __syncwarp();
-        gather<FWD>(a, t, children, lane, 32, v);
+        gather<FWD>(a, t, children, root, lane, 32, v);
         __syncwarp();
         const int L = t.n_out > 32 ? 32 : t.n_out > 16 ? 16 : 8;  // lanes across the outputs, two each
         const int R = 32 / L, sub = lane / L, ol = 2 * (lane & (L - 1));
@@ -255,17 +257,25 @@ __global__ void __launch_bounds__(kNdThreads, kNdPerSm) k_nd_solve(const __grid_
     extern __shared__ __align__(16) double vec[];
     __shared__ __align__(16) double red[2 * kNdThreads];  // (split of the inputs) x width
     cooperative_groups::grid_group grid = cooperative_groups::this_grid();
-    for (int i = blockIdx.x * kNdThreads + threadIdx.x; i < a.nd.n_outside; i += gridDim.x * kNdThreads)
-        a.phi[a.nd.outside[i]] = 0.0;
     for (int k = a.nd.n_levels - 1; k >= 0; --k) {
         const oec_nd_level_t &l = a.nd.level[k];
         run_level<true>(a, l.fwd, l.has_children != 0, k == 0, vec, red);
         if (a.nd.n_levels > 1) grid.sync();
     }
+    // phi is written from the root on, when q has been read (it may be the same memory)
+    for (int i = blockIdx.x * kNdThreads + threadIdx.x; i < a.nd.n_outside; i += gridDim.x * kNdThreads)
+        a.phi[a.nd.outside[i]] = 0.0;
     for (int k = 1; k < a.nd.n_levels; ++k) {
         run_level<false>(a, a.nd.level[k].bwd, false, false, vec, red);
         if (k + 1 < a.nd.n_levels) grid.sync();
     }
+}
+
+// q on the pivots into y, before a solve whose q and phi share memory: the tiles of
+// the root read q while others of them write phi.  (The fronts below overwrite their
+// part of y, and have read q before anything of phi is written.)
+__global__ void k_nd_stage(int n, const int32_t *__restrict__ piv_node, const double *q, double *__restrict__ y) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) y[i] = q[piv_node[i]];
 }
 
 // A pass fits the kernel: its tiles exist, its group is one of the three and its
@@ -305,7 +315,13 @@ int nd_solve(const oec_nd_t *nd, const double *q, double *phi, double *work, cud
                    : 0;
     });
     if (!ok) return OEC_ERR_CUDA;
-    NdArgs a{*nd, q, phi, work, work + nd->n};
+    const uintptr_t q0 = reinterpret_cast<uintptr_t>(q), p0 = reinterpret_cast<uintptr_t>(phi);
+    const uintptr_t bytes = sizeof(double) * (uintptr_t)nd->n_nodes;
+    NdArgs a{*nd, q, phi, work, work + nd->n, q0 < p0 + bytes && p0 < q0 + bytes};
+    if (a.staged) {
+        k_nd_stage<<<persistent_grid((nd->n + 255) / 256, 4), 256, 0, s>>>(nd->n, nd->piv_node, q, a.y);
+        OEC_LAUNCH_CHECK();
+    }
     if (nd->n_levels == 1) {  // no barrier: an ordinary launch
         k_nd_solve<<<(unsigned)need, kNdThreads, smem, s>>>(a);
         OEC_LAUNCH_CHECK();

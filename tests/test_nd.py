@@ -129,3 +129,34 @@ def test_solve_on_a_part_of_the_device(gpu, p):
         s.phi.fill_(-1.0)
         s.solve(q)
         assert np.array_equal(s.getPhi(), x), ctas
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("levels", ["model", "many"])
+@pytest.mark.parametrize("p", GRIDS + [(402, 301, 0.09, 0.036, 1)])
+def test_solve_over_its_own_charge(gpu, p, levels, monkeypatch):
+    """phi in the charge's memory, and shifted against it both ways: the bits of a solve into
+    an array of its own."""
+    import ctypes
+    import torch
+    from openecloud_b200 import device as D
+    from openecloud_b200 import nd_setup
+    from openecloud_b200.poissonSolver import PoissonSolver, _declare
+    if levels == "many":
+        for k in ("PHASE_US", "TILE_US", "GATHER_US", "BLOCK_US", "WARP_US"):
+            monkeypatch.setattr(nd_setup, k, 0.0)
+    g, a, inside, q, *_ = _case(p)
+    ps = PoissonSolver(g)
+    ps.solve(q)
+    want = ps.getPhi()
+    ps.phi.copy_(torch.as_tensor(q))
+    ps.solveDevice(ps.getPhiDevice())
+    assert np.array_equal(ps.getPhi(), want)
+    n = q.size
+    for shift in (-g.getNxExt(), -1, 1, n // 2, n - 1):
+        buf = D.zeros(3 * n, torch.float64)
+        buf[n:2 * n] = torch.as_tensor(q, device="cuda")
+        phi = buf[n + shift:2 * n + shift]
+        rc = _declare().oec_lu_solve(ctypes.byref(ps._lu_t), buf[n:].data_ptr(), phi.data_ptr(), ps._work.data_ptr(),
+                                     D.stream())
+        assert rc == 0 and np.array_equal(phi.cpu().numpy(), want), shift
