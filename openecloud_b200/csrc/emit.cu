@@ -743,8 +743,9 @@ extern "C" int oec_furman_emit(const oec_furman_t *params, const double *rows_de
         return OEC_ERR_INVALID;
     if (cap > kMaxAbsorbedRows) return OEC_ERR_INVALID;
     cudaStream_t s = as_stream(stream);
-    // work layout: SplitConst | Rec[cap] | split[cap * kSlots] (f64) | tile_sum[cap / kTileRows]
-    char *w = static_cast<char *>(work_dev);
+    // work layout: SplitConst | Rec[cap] | split[cap * kSlots] (f64) | tile_sum[cap / kTileRows], from the
+    // first multiple of 16 bytes on (SplitConst is read 16 bytes at a time; the work bytes have the slack)
+    char *w = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(work_dev) + 15) & ~uintptr_t(15));
     SplitConst *consts = reinterpret_cast<SplitConst *>(w);
     Rec *rec = reinterpret_cast<Rec *>(w + sizeof(SplitConst));
     double *split = reinterpret_cast<double *>(rec + cap);

@@ -63,3 +63,38 @@ def test_all_secondary_counts_match_oracle(gpu, material, sey, n):
         assert np.max(np.abs(sec[:, 2:5] - ref[:, 2:5])) <= 1e-10 * np.max(np.abs(ref[:, 2:5]))
     if n > 20000 and material == "copper" and sey > 5:
         assert len(sec) > 60000  # many counts above one
+
+
+@pytest.mark.parametrize("shift", [8, 16, 24])
+def test_work_area_at_any_eight_bytes(gpu, shift):
+    """A work area of the stated size that starts at any multiple of 8 bytes gives the
+    rows of one from the allocator, and nothing behind its end is written."""
+    import torch
+    from openecloud_b200.grid import Grid
+    from openecloud_b200.particleBoundary import AbsorbElliptical
+    from openecloud_b200.particleEmitter import FurmanEmitter
+    from openecloud_b200.particles import Particles
+    n = 1025
+    rows, nv = _rows(n, 5)
+    P = Particles("electrons", "variableWeight")
+    P.setParticleData(np.zeros((0, 6)))
+    g = Grid(64, 64, 0.04, 0.04, 1)
+    P._bind(g)
+    bd = AbsorbElliptical(g, P)
+    bd.ensure_buffers(n)
+    bd._rows[:n] = torch.as_tensor(rows, device="cuda")
+    bd._normals[:n] = torch.as_tensor(nv, device="cuda")
+    bd._n_abs.fill_(n)
+    bd._index = None
+    bd._wall_done = True
+    bd.absorbedMacroParticleCount = n
+    em = FurmanEmitter(bd, P, seyMax=6.0, seed=7)
+    u = torch.as_tensor(np.random.default_rng(n).random((n, 32)), device="cuda")
+    want = em.generateSecondaries(replay=u).clone()
+    size = em._work.shape[0]
+    area = torch.full((size + 64,), 0x5a, dtype=torch.uint8, device="cuda")
+    em._work = area[shift:shift + size]
+    em._out.fill_(0.0)
+    got = em.generateSecondaries(replay=u)
+    assert len(want) > n and torch.equal(got, want)
+    assert bool((area[:shift] == 0x5a).all()) and bool((area[shift + size:] == 0x5a).all())
