@@ -396,8 +396,15 @@ int oec_roulette_select(int32_t n, int32_t n_remove, uint32_t *mask_dev, int64_t
 int oec_clone_rows(const oec_grid_t *grid, const oec_particles_t *p, int32_t n, int32_t k, uint64_t seed,
                    uint32_t call, double *rows_dev, void *stream);
 
-/* acc_dev[0] = sum w, acc_dev[1] = sum |v|^2 w^2 (localRandom :124-128). */
+/* acc_dev[0] = sum w, acc_dev[1] = sum |v|^2 w^2 (localRandom :124-128), the
+ * parts added in the order of their arrival. */
 int oec_weight_stats(const oec_particles_t *p, double *acc_dev, void *stream);
+
+/* The same sums in an order that follows from the particle count (on one kind
+ * of device the same bits from call to call and for any capacity).
+ * scratch_dev: 2 * OEC_WEIGHT_SUMS_CTAS doubles. */
+#define OEC_WEIGHT_SUMS_CTAS 1024
+int oec_weight_sums(const oec_particles_t *p, double *acc_dev, double *scratch_dev, void *stream);
 
 /* Halve the weights of the last k of the first n particles and write their
  * duplicates as rows (localRandom split, particleManagement.pyx:130-163). */

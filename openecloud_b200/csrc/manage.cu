@@ -366,12 +366,19 @@ __global__ void k_clone_rows(oec_particles_t p, int n, int k, uint2 key, uint32_
 
 // ------------------------------------------------------------ local merge
 
-// Stats over particles [0, n): sum w, sum |v|^2 w^2 (f64, one atomic per sum and CTA).
-__global__ void k_wstats(oec_particles_t p, double *acc) {
-    __shared__ double sh[2][32];
-    int n = *p.count;
+// Sums over a store's particles, sum w and sum |v|^2 w^2 (f64): those of one CTA, in
+// threads 0 and 1.  Which CTA takes which particles depends on their number alone.
+constexpr int kStatThreads = 256, kStatCtas = OEC_WEIGHT_SUMS_CTAS;
+
+// CTAs with particles, of at most `ctas`.
+__device__ __forceinline__ int stat_ctas(int n, int ctas) {
+    return (int)min((int64_t)ctas, ((int64_t)n + kStatThreads - 1) / kStatThreads);
+}
+
+__device__ __forceinline__ double stat_cta(const oec_particles_t &p, int n) {
+    __shared__ double sh[2][kStatThreads / 32];
     double sw = 0, sv = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    for (int i = blockIdx.x * kStatThreads + threadIdx.x; i < n; i += stat_ctas(n, gridDim.x) * kStatThreads) {
         double w = p.w[i], vx = p.vx[i], vy = p.vy[i], vz = p.vz[i];
         sw += w;
         sv += (vx * vx + vy * vy + vz * vz) * w * w;
@@ -385,11 +392,38 @@ __global__ void k_wstats(oec_particles_t p, double *acc) {
         sh[1][threadIdx.x >> 5] = sv;
     }
     __syncthreads();
-    if (threadIdx.x < 2) {
-        double t = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sh[threadIdx.x][w];
-        atomicAdd(&acc[threadIdx.x], t);
-    }
+    double t = 0;
+    if (threadIdx.x < 2)
+        for (int w = 0; w < kStatThreads / 32; ++w) t += sh[threadIdx.x][w];
+    return t;
+}
+
+// Added to acc, one atomic per sum and CTA: in the order of arrival.
+__global__ void __launch_bounds__(kStatThreads) k_wstats(oec_particles_t p, double *acc) {
+    const int n = *p.count;
+    if ((int)blockIdx.x >= stat_ctas(n, gridDim.x)) return;
+    const double t = stat_cta(p, n);
+    if (threadIdx.x < 2) atomicAdd(&acc[threadIdx.x], t);
+}
+
+// Left in part (all of sum w, then all of sum |v|^2 w^2) for k_wsums.
+__global__ void __launch_bounds__(kStatThreads) k_wparts(oec_particles_t p, double *part) {
+    const int n = *p.count;
+    if ((int)blockIdx.x >= stat_ctas(n, gridDim.x)) return;
+    const double t = stat_cta(p, n);
+    if (threadIdx.x < 2) part[threadIdx.x * kStatCtas + blockIdx.x] = t;
+}
+
+// The CTAs' sums in a fixed order, a warp per sum.  The thresholds of a merge follow
+// from them, so that two runs of one store must agree to the last bit.
+__global__ void __launch_bounds__(64) k_wsums(const int32_t *count, int ctas, const double *__restrict__ part,
+                                              double *__restrict__ acc) {
+    const int parts = stat_ctas(*count, ctas);
+    const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+    double t = 0;
+    for (int i = lane; i < parts; i += 32) t += part[k * kStatCtas + i];
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(kFullMask, t, o);
+    if (lane == 0) acc[k] = t;
 }
 
 struct MergeArgs {
@@ -721,7 +755,17 @@ extern "C" int oec_weight_stats(const oec_particles_t *p, double *acc_dev, void 
     if (!vp2(p) || !acc_dev) return OEC_ERR_INVALID;
     cudaStream_t s = as_stream(stream);
     OEC_CUDA_TRY(cudaMemsetAsync(acc_dev, 0, 2 * sizeof(double), s));
-    k_wstats<<<persistent_grid((p->capacity + 255) / 256, 4), 256, 0, s>>>(*p, acc_dev);
+    k_wstats<<<persistent_grid((p->capacity + kStatThreads - 1) / kStatThreads, 4), kStatThreads, 0, s>>>(*p, acc_dev);
+    OEC_LAUNCH_CHECK();
+    return OEC_OK;
+}
+
+extern "C" int oec_weight_sums(const oec_particles_t *p, double *acc_dev, double *scratch_dev, void *stream) {
+    if (!vp2(p) || !acc_dev || !scratch_dev) return OEC_ERR_INVALID;
+    cudaStream_t s = as_stream(stream);
+    const int ctas = std::min(persistent_grid((p->capacity + kStatThreads - 1) / kStatThreads, 4), kStatCtas);
+    k_wparts<<<ctas, kStatThreads, 0, s>>>(*p, scratch_dev);
+    k_wsums<<<1, 64, 0, s>>>(p->count, ctas, scratch_dev, acc_dev);
     OEC_LAUNCH_CHECK();
     return OEC_OK;
 }

@@ -21,6 +21,8 @@ from . import _lib
 from . import device as D
 from .constants import c
 
+WEIGHT_SUMS_CTAS = 1024  # OEC_WEIGHT_SUMS_CTAS: places per sum in the scratch of oec_weight_sums
+
 _CALLS = {"n": 0}
 
 
@@ -73,10 +75,11 @@ def localRandom(gridObj, particlesObj, particleBoundaryObj, targetMacroParticleC
     n = P.getMacroParticleCount()
     target = int(targetMacroParticleCount)
     s = D.stream()
-    # both sums at once, before the sort (they do not depend on the order)
-    acc = D.zeros(2, torch.float64)
-    _lib.call("oec_weight_stats", P.c_particles(), acc.data_ptr(), s)
-    sum_w, sum_v2w2 = (float(x) for x in D.to_numpy(acc))
+    # both sums at once, in an order that follows from the count: the thresholds and with
+    # them the particles merged and split are the same in every run of the same store
+    sums = D.empty(2 + 2 * WEIGHT_SUMS_CTAS, torch.float64)
+    _lib.call("oec_weight_sums", P.c_particles(), sums.data_ptr(), sums[2:].data_ptr(), s)
+    sum_w, sum_v2w2 = (float(x) for x in D.to_numpy(sums[:2]))
     meanWeight = sum_w / n
     goal = meanWeight * n / target
     maxT, minT = thresholdFactor * goal, goal / thresholdFactor

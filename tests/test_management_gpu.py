@@ -217,3 +217,67 @@ def test_weight_thresholds_match_reference_search(gpu):
         _lib.call("oec_weight_thresholds", P.c_particles(), float(lo), float(hi), thr.data_ptr(), D.stream())
         got = tuple(int(x) for x in D.to_numpy(thr))
         assert got == (_search_sorted_ref(w, lo), _search_sorted_ref(w, hi)), (lo, hi, got)
+
+
+def test_local_random_repeats_bit_for_bit(gpu):
+    """A merge of the same store gives the same rows every time, also where a sixth of the
+    weights equals the merge threshold up to the last bit of the mean weight."""
+    from openecloud_b200.grid import Grid
+    from openecloud_b200.particleBoundary import AbsorbElliptical
+    from openecloud_b200.particleManagement import localRandom
+    from openecloud_b200.particles import Particles
+    rng = np.random.default_rng(12)
+    n = 600_001
+    pd = np.empty((n, 6))
+    pd[:, 0:2] = rng.uniform(-0.012, 0.012, (n, 2))
+    pd[:, 2:5] = rng.normal(0, 1e6, (n, 3))
+    pd[:, 5] = rng.uniform(0.5, 2.0, n)
+    pd[::6, 5] = 0.5
+    pd[1::5, 5] = 10 ** rng.uniform(-9, -1, pd[1::5].shape[0])  # sums of these round
+    pd[:, 5] = pd[:, 5].astype(np.float32)
+    g = Grid(64, 64, 0.04, 0.04, 1)
+    target = n - n // 10
+    goal = pd[:, 5].sum() / target
+    first = None
+    for k in range(12):
+        P = Particles("electrons", "variableWeight", capacity=n + 50_000 * (k % 3))
+        P.setParticleData(pd)
+        P._bind(g)
+        localRandom(g, P, AbsorbElliptical(g, P), target, thresholdFactor=goal / 0.5, seed=3, call=1)
+        rows = P.getParticleData()
+        first = rows if first is None else first
+        assert np.array_equal(rows, first), k
+
+
+@pytest.mark.parametrize("n", [0, 1, 33, 255, 257, 600_001])
+def test_weight_sums(gpu, n):
+    """Both sums, against exact ones: at most 2e-14 apart (a thread adds up to 5 terms, a
+    CTA 256 threads in 13 additions, the last warp up to 19 sums of CTAs and 5 more: less
+    than 60 roundings of one sign), with the same bits for every capacity."""
+    import math
+    import torch
+    from openecloud_b200 import _lib
+    from openecloud_b200 import device as D
+    from openecloud_b200.grid import Grid
+    from openecloud_b200.particles import Particles
+    rng = np.random.default_rng(n)
+    pd = np.zeros((n, 6))
+    pd[:, 2:5] = rng.normal(0, 1e6, (n, 3))
+    pd[:, 5] = 10 ** rng.uniform(-3, 3, n)
+    got = []
+    for cap in (n, 2 * n + 5000, 3_000_000):
+        P = Particles("electrons", "variableWeight", capacity=cap)
+        P.setParticleData(pd)
+        P._bind(Grid(32, 32, 0.04, 0.04, 0))
+        acc = torch.full((2,), 9.0, dtype=torch.float64, device="cuda")
+        scratch = torch.full((2048,), float("nan"), dtype=torch.float64, device="cuda")
+        _lib.call("oec_weight_sums", P.c_particles(), acc.data_ptr(), scratch.data_ptr(), D.stream())
+        got.append(acc.cpu().numpy())
+        old = torch.full((2,), 9.0, dtype=torch.float64, device="cuda")
+        _lib.call("oec_weight_stats", P.c_particles(), old.data_ptr(), D.stream())
+        assert np.allclose(old.cpu().numpy(), got[0], rtol=4e-14, atol=0)
+    s = P.soa()
+    w, v = s["w"][:n].cpu().numpy().astype(np.float64), [s[k][:n].cpu().numpy().astype(np.float64) for k in ("vx", "vy", "vz")]
+    want = math.fsum(w), math.fsum((v[0] ** 2 + v[1] ** 2 + v[2] ** 2) * w * w)
+    assert all(np.array_equal(x, got[0]) for x in got)
+    assert np.allclose(got[0], want, rtol=2e-14, atol=0)
