@@ -113,8 +113,15 @@ class BatchedBuildup:
 
     def _capture(self, nb):
         nodes = [b.ps.n_nodes for b in self.runs]
-        for _, ps in self.shared.values():
-            ps.shareSolve(solve_ctas(ps.n_nodes, sum(nodes) / len(nodes), nb))
+        before = [(ps, ps.shareSolve(solve_ctas(ps.n_nodes, sum(nodes) / len(nodes), nb)))
+                  for _, ps in self.shared.values()]
+        try:
+            self._capture_step(nb)
+        finally:  # the graph keeps its parts; a run solved by itself later has the whole device
+            for ps, ctas in before:
+                ps.shareSolve(ctas)
+
+    def _capture_step(self, nb):
         for b in self.runs:
             b.ps.prepare()
         while len(self._streams) < nb:

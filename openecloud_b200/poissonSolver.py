@@ -369,9 +369,12 @@ class PoissonSolver:
 
     def shareSolve(self, ctas):
         """At most `ctas` CTAs (0: all that fit) for each direct solve from now
-        on, of this solver and its siblings.  The results do not depend on it."""
-        if self._lu_t.nd:
-            self._nd_t.ctas = int(ctas)
+        on, of this solver and its siblings (a captured one keeps what it was
+        captured with).  Returns the limit before.  The results do not depend on it."""
+        if not self._lu_t.nd:
+            return 0
+        before, self._nd_t.ctas = self._nd_t.ctas, int(ctas)
+        return before
 
     def applyOperator(self, x):
         """A x on the inside nodes (device f64 [npExt] in and out)."""

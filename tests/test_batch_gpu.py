@@ -80,6 +80,19 @@ def test_batched_multigrid_runs_and_autotuner(gpu):
         assert b.ps.nFallbacks == 0 and b.ps.lastStats.converged == 1 and b.ps.lastStats.rel_residual <= 1e-8
 
 
+@pytest.mark.gpu
+def test_batch_leaves_the_whole_device_to_later_solves(gpu):
+    """The part of the device that a batch gives each of its solves is part of its graph
+    alone: afterwards a solver has the limit it had before."""
+    from openecloud_b200.batch import BatchedBuildup
+    batch = BatchedBuildup([dict(r, n_steps_table=30) for r in RUNS], branches=4, poisson="lu")
+    solvers = [ps for _, ps in batch.shared.values()]
+    assert [ps._nd_t.ctas for ps in solvers] == [0, 0]
+    solvers[1].shareSolve(100)
+    batch.run(3)
+    assert [ps._nd_t.ctas for ps in solvers] == [0, 100]
+
+
 def test_shard_runs_balances_and_covers():
     from openecloud_b200.batch import run_cost, scan_configs, shard_runs
     runs = scan_configs(64)
