@@ -3,12 +3,12 @@
 Every choice is made by timing the candidates on the GPU the run uses (CUDA
 events) on the run's own grid, and remembered per key for the process (and in
 a JSON file when a path is given, so a scan of many runs measures each key
-once):
+once; timings of other kernels than these are measured anew):
 
-* Poisson solve per grid: the LU back-substitution against the
+* Poisson solve per grid: the direct solve against the
   multigrid-preconditioned iterative solve at the solver's tolerance, timed
   warm-started as in a time step (the previous step's phi of a 0.1 %-different
-  charge); a tie keeps LU (it is exact without iterating).
+  charge); a tie keeps the direct one (it is exact without iterating).
 * Multigrid block size per grid: the largest level (nodes) handed to the
   one-CTA shared-memory solve of the V-cycle (a tile of the hierarchy): small
   blocks give the coarse levels to the tiled kernels (more launches), large
@@ -28,6 +28,11 @@ import torch
 from . import device as D
 
 MG_BLOCK_TOPS = (320, 1280, 4608, 9000)
+
+# Goes up when kernels that the choices compare have changed: measurements of another
+# version say nothing about this one (before the direct solve ran on fronts "mg" won on
+# large grids, where it is now 4 to 9 times slower).
+VERSION = 2
 
 
 def _time(fn, reps):
@@ -71,7 +76,14 @@ class Autotuner:
         self.choices = {}
         if path and os.path.exists(path):
             with open(path) as f:
-                self.choices = json.load(f)
+                known = json.load(f)
+            # a choice without timings was put there by hand and stays
+            self.choices = {k: v for k, v in known.items() if not isinstance(v, dict) or v.get("version") == VERSION
+                            or not any(t.startswith("ms_per_") for t in v)}
+
+    def _remember(self, key, **entry):
+        self.choices[key] = dict(entry, version=VERSION)
+        self._save()
 
     def _save(self):
         if self.path:
@@ -101,8 +113,7 @@ class Autotuner:
                 times[str(top)] = _time(lambda: L.oec_mg_apply(ctypes.byref(c), r.data_ptr(), z.data_ptr(),
                                                                 D.stream()), 4 * self.reps)
             best = min(times, key=times.get)
-            self.choices[key] = {"choice": int(best), "ms_per_vcycle": times}
-            self._save()
+            self._remember(key, choice=int(best), ms_per_vcycle=times)
         top = self.choices[key]["choice"]
         ps._mg_setup(block_top=top)
         return top
@@ -127,8 +138,7 @@ class Autotuner:
             times["mg"] = _time(warm, self.reps) / 2.0
             ps.method, ps.precond, ps.warmStart = saved
             best = "mg" if times["mg"] < times["lu"] else "lu"
-            self.choices[key] = {"choice": best, "ms_per_solve": times}
-            self._save()
+            self._remember(key, choice=best, ms_per_solve=times)
         best = self.choices[key]["choice"]
         if best == "mg":
             ps.method, ps.precond = "pcg", "mg"
@@ -142,6 +152,5 @@ class Autotuner:
         if key not in self.choices:
             times = {str(c): trial(c) for c in candidates}
             best = min(times, key=times.get)
-            self.choices[key] = {"choice": int(best), "ms_per_step": times}
-            self._save()
+            self._remember(key, choice=int(best), ms_per_step=times)
         return self.choices[key]["choice"]

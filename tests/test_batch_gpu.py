@@ -38,6 +38,18 @@ def test_autotuner_keeps_fastest_and_records(tmp_path):
     assert Autotuner(path=str(path)).branches("k", [1], trial) == 4  # read back from the file
 
 
+def test_autotuner_measures_anew_what_other_kernels_were_timed_for(tmp_path):
+    from openecloud_b200.autotune import Autotuner
+    path = tmp_path / "tune.json"
+    path.write_text(json.dumps({"branches/old": {"choice": 16, "ms_per_step": {"1": 2.0, "16": 1.0}},
+                                "branches/pinned": {"choice": 4}}))
+    t = Autotuner(path=str(path))
+    assert t.branches("old", [1, 16], lambda c: float(c)) == 1
+    assert t.branches("pinned", [1, 16], lambda c: float(c)) == 4
+    again = Autotuner(path=str(path))
+    assert again.choices == t.choices and again.branches("old", [1, 16], lambda c: -float(c)) == 1
+
+
 @pytest.mark.gpu
 def test_batched_run_equals_standalone_run(gpu):
     from openecloud_b200.batch import BatchedBuildup
