@@ -224,9 +224,8 @@ class PoissonSolver:
 
     def __init__(self, gridObj, tail=None, method="lu", precond="jacobi", pcgTol=1e-8, pcgMaxIter=4000,
                  warmStart="extrapolate", factors=None):
-        """factors: the result of lu_setup.factor(gridObj) when the host
-        setup (assembly and SuperLU factorisation) was done beforehand, e.g.
-        for several grids in parallel threads."""
+        """factors: the result of lu_setup.factor(gridObj) when the assembly
+        was done beforehand, e.g. for several grids in parallel threads."""
         nx = gridObj.getNxExt()
         npn = gridObj.getNpExt()
         self.gridObj = gridObj
