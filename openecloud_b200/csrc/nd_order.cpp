@@ -10,6 +10,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <new>
 #include <vector>
 
 #include "oec.h"
@@ -24,9 +25,8 @@ struct Piece {
 
 }  // namespace
 
-extern "C" int oec_nd_dissect(int64_t n, const int32_t *ix, const int32_t *iy, int32_t max_depth, int32_t leaf,
-                              int64_t *node_out) {
-    if (n <= 0 || !ix || !iy || !node_out || max_depth < 0 || max_depth > 40 || leaf < 1) return OEC_ERR_INVALID;
+static void dissect(int64_t n, const int32_t *ix, const int32_t *iy, int32_t max_depth, int32_t leaf,
+                    int64_t *node_out) {
     std::vector<int32_t> idx((size_t)n), count;
     for (int64_t i = 0; i < n; ++i) idx[(size_t)i] = (int32_t)i;
     std::vector<Piece> todo;
@@ -43,9 +43,10 @@ extern "C" int oec_nd_dissect(int64_t n, const int32_t *ix, const int32_t *iy, i
             y0 = std::min(y0, iy[*k]);
             y1 = std::max(y1, iy[*k]);
         }
-        const bool along_x = x1 - x0 >= y1 - y0;
+        const int64_t lx = (int64_t)x1 - x0, ly = (int64_t)y1 - y0;
+        const bool along_x = lx >= ly;
         const int32_t *c = along_x ? ix : iy;
-        const int32_t lo = along_x ? x0 : y0, len = (along_x ? x1 - x0 : y1 - y0) + 1;
+        const int64_t lo = along_x ? x0 : y0, len = (along_x ? lx : ly) + 1;
         if (p.depth >= max_depth || m <= leaf || len < 3) {
             for (int32_t *k = a; k < b; ++k) node_out[*k] = p.node;
             continue;
@@ -54,7 +55,7 @@ extern "C" int oec_nd_dissect(int64_t n, const int32_t *ix, const int32_t *iy, i
         count.assign((size_t)len, 0);
         for (int32_t *k = a; k < b; ++k) ++count[(size_t)(c[*k] - lo)];
         int64_t below = 0, best = -1, best_cost = 0;
-        for (int32_t l = 0; l < len; ++l) {
+        for (int64_t l = 0; l < len; ++l) {
             const int64_t here = count[(size_t)l], above = m - below - here;
             const int64_t cost = 4 * std::max(below, above) + here;
             if (best < 0 || cost < best_cost) {
@@ -63,12 +64,23 @@ extern "C" int oec_nd_dissect(int64_t n, const int32_t *ix, const int32_t *iy, i
             }
             below += here;
         }
-        const int32_t cut = lo + (int32_t)best;
+        const int32_t cut = (int32_t)(lo + best);
         int32_t *u = std::partition(a, b, [&](int32_t i) { return c[i] < cut; });
         int32_t *v = std::partition(u, b, [&](int32_t i) { return c[i] == cut; });
         for (int32_t *k = u; k < v; ++k) node_out[*k] = p.node;
         if (u > a) todo.push_back({p.first, p.first + (u - a), 2 * p.node, p.depth + 1});
         if (b > v) todo.push_back({p.first + (v - a), p.last, 2 * p.node + 1, p.depth + 1});
+    }
+}
+
+extern "C" int oec_nd_dissect(int64_t n, const int32_t *ix, const int32_t *iy, int32_t max_depth, int32_t leaf,
+                              int64_t *node_out) {
+    if (n <= 0 || n > INT32_MAX || !ix || !iy || !node_out || max_depth < 0 || max_depth > 40 || leaf < 1)
+        return OEC_ERR_INVALID;
+    try {
+        dissect(n, ix, iy, max_depth, leaf, node_out);
+    } catch (const std::bad_alloc &) {
+        return OEC_ERR_HOST;
     }
     return OEC_OK;
 }

@@ -160,3 +160,27 @@ def test_solve_over_its_own_charge(gpu, p, levels, monkeypatch):
         rc = _declare().oec_lu_solve(ctypes.byref(ps._lu_t), buf[n:].data_ptr(), phi.data_ptr(), ps._work.data_ptr(),
                                      D.stream())
         assert rc == 0 and np.array_equal(phi.cpu().numpy(), want), shift
+
+
+def test_dissection_without_the_memory_for_it_returns_an_error():
+    """No exception crosses the C entry: positions that span two thousand million lines (the
+    counts per line take 8 GB) in a process that may not have that, and more unknowns than
+    an index has, give a status; the spans at the ends of int32 are told right."""
+    import subprocess
+    import sys
+    code = """
+import ctypes, resource
+import numpy as np
+from openecloud_b200 import _lib, nd_setup
+L, p = nd_setup._declare(), lambda a: a.ctypes.data_as(ctypes.c_void_p)
+out = np.zeros(4, np.int64)
+far = np.array([0, 2 ** 31 - 2, 5, 9], np.int32)
+ends = np.array([-2 ** 31, 2 ** 31 - 1, 5, 9], np.int32)
+zero = np.zeros(4, np.int32)
+resource.setrlimit(resource.RLIMIT_AS, (3 << 30, 3 << 30))
+print(L.oec_nd_dissect(4, p(far), p(zero), 3, 1, p(out)), L.oec_nd_dissect(4, p(ends), p(zero), 3, 1, p(out)),
+      L.oec_nd_dissect(2 ** 31, p(far), p(zero), 3, 1, p(out)), L.oec_nd_dissect(4, p(zero), p(zero), 3, 1, p(out)))
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-500:]
+    assert r.stdout.split() == ["6", "6", "1", "0"]  # OEC_ERR_HOST, OEC_ERR_INVALID, OEC_OK
