@@ -98,3 +98,9 @@ def test_work_area_at_any_eight_bytes(gpu, shift):
     got = em.generateSecondaries(replay=u)
     assert len(want) > n and torch.equal(got, want)
     assert bool((area[:shift] == 0x5a).all()) and bool((area[shift + size:] == 0x5a).all())
+
+
+def test_second_chunks_match_oracle(gpu):
+    """More rows than all CTAs take as their first chunk (2 x 148 x 1024): the places of a
+    second chunk's secondaries follow from the sums of the rows between."""
+    test_all_secondary_counts_match_oracle(gpu, "copper", 1.6, 320_001)

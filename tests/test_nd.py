@@ -184,3 +184,61 @@ print(L.oec_nd_dissect(4, p(far), p(zero), 3, 1, p(out)), L.oec_nd_dissect(4, p(
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr[-500:]
     assert r.stdout.split() == ["6", "6", "1", "0"]  # OEC_ERR_HOST, OEC_ERR_INVALID, OEC_OK
+
+
+QUARTERS = [(150, 120, 0.09, 0.036, 0), (192, 192, 0.04, 0.04, 1), (300, 240, 0.044, 0.036, 0)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("p", QUARTERS)
+def test_tiles_by_quarters_of_a_cta(gpu, p):
+    """Grids whose lowest level goes to groups of 128 threads: the whole device, and parts of
+    it that leave several tiles to a group, give the same bits."""
+    from openecloud_b200.poissonSolver import PoissonSolver
+    g, a, inside, q, phi, tol = _case(p)
+    ps = PoissonSolver(g)
+    low = ps._nd_t.level[ps._nd_t.n_levels - 1]
+    assert low.fwd.group == 128 and low.fwd.tiles > 600
+    ps.solve(q)
+    x = ps.getPhi()
+    assert np.linalg.norm(x - phi) <= tol * np.linalg.norm(phi)
+    for ctas in (1, 7, 74, 148):
+        ps.shareSolve(ctas)
+        ps.phi.fill_(-1.0)
+        ps.solve(q)
+        assert np.array_equal(ps.getPhi(), x), ctas
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("p", [(96, 96, 0.04, 0.04, 1), (200, 131, 0.06, 0.05, 1), (512, 512, 0.09, 0.036, 1)])
+def test_device_keeps_the_accuracy_of_row_sums(gpu, p):
+    """test_fronts_keep_the_accuracy_of_row_sums with the blocks inverted on the device and
+    the solve made there, up to 512^2: the same 64 eps."""
+    from openecloud_b200.poissonSolver import PoissonSolver
+    g, a, inside, q, *_ = _case(p)
+    q = np.abs(q)
+    csr, lu = a.tocsr(), spla.splu(a.tocsc())
+    x = lu.solve(q[inside]).astype(np.longdouble)
+    for _ in range(4):
+        r = q[inside] - np.add.reduceat(csr.data.astype(np.longdouble) * x[csr.indices], csr.indptr[:-1])
+        x += lu.solve(r.astype(np.float64))
+    ps = PoissonSolver(g)
+    ps.solve(q)
+    d = ps.getPhi()[inside] - x
+    assert np.sqrt((d * d).sum()) <= 64 * 2.3e-16 * np.sqrt((x * x).sum())
+
+
+def test_front_structures_follow_the_header(tmp_path, monkeypatch):
+    """The ctypes structures of the fronts, and the numpy records of their tiles, have the
+    layout of include/oec.h."""
+    import ctypes
+    import test_abi_layout
+    from openecloud_b200 import nd_setup
+    ct = {np.dtype(np.int64): ctypes.c_int64, np.dtype(np.int32): ctypes.c_int32}
+    Tile = type("Tile", (ctypes.Structure,), {"_fields_": [(k, ct[nd_setup.TILE[k]]) for k in nd_setup.TILE.names]})
+    assert ctypes.sizeof(Tile) == nd_setup.TILE.itemsize
+    assert all(getattr(Tile, k).offset == nd_setup.TILE.fields[k][1] for k in nd_setup.TILE.names)
+    classes = {"oec_nd_pass_t": nd_setup.NdPass_t, "oec_nd_level_t": nd_setup.NdLevel_t, "oec_nd_t": nd_setup.Nd_t,
+               "oec_nd_tile_t": Tile}
+    monkeypatch.setattr(test_abi_layout, "_classes", lambda: classes)
+    test_abi_layout.test_ctypes_structures_follow_the_header(tmp_path)

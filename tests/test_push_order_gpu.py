@@ -112,3 +112,44 @@ def test_chunks_at_the_limit_of_the_deposit_choice(gpu, rows_apart):
 
     got, want = step(rows), step(rows[rng.permutation(n)])
     assert want[0].any() and all(torch.equal(x, want[0]) for x in got + want)
+
+
+@pytest.mark.parametrize("bound,btype", [(0, 0), (1, 1)])
+def test_several_chunks_per_cta(gpu, bound, btype):
+    """More chunks than resident CTAs (four on each of 148 SMs), in random and in cell order."""
+    test_random_and_cell_order_agree(gpu, 700_001, bound, btype)
+
+
+@pytest.mark.parametrize("btype", [0, 2])
+@pytest.mark.parametrize("n", [1025, 500_001])
+def test_cut_cells_and_uneven_weights(gpu, n, btype):
+    """The cut-cell wall (three CTAs per SM, 500,001 electrons are more chunks than those)
+    with weights from 1e-9 to 1, so that charges lie on both sides of the 2^40 up to which
+    the windows take them without a test: both orders agree and the deposit is exact."""
+    import torch
+    from openecloud_b200.grid import Grid
+    from openecloud_b200.particleBoundary import AbsorbArbitraryCutCell
+    from openecloud_b200.particles import Particles
+    rng = np.random.default_rng(n)
+    rows = np.empty((n, 6))
+    rows[:, 0], rows[:, 1] = rng.uniform(-0.0199, 0.0199, n), rng.uniform(-0.0299, 0.0299, n)
+    rows[:, 2:5] = rng.normal(0, 2e6, (n, 3))
+    rows[:, 5] = 10 ** rng.uniform(-9, 0, n)
+    order = np.lexsort((rows[:, 0], np.floor(rows[:, 1] / (0.06 / 219))))
+    g = Grid(150, 220, 0.04, 0.06, 1)
+    e = np.random.default_rng(1).normal(0, 1e4, 2 * g.getNpExt())
+    b = np.random.default_rng(2).normal(0, 0.1, 3 * g.getNpExt())
+    got = []
+    for r in (rows, rows[order]):
+        P = Particles("electrons", "variableWeight")
+        P.setParticleData(r)
+        P._bind(g)
+        tabs = P.fieldTable(g, e, 2), P.fieldTable(g, b, 3) if btype == 2 else None
+        P.pushGatherDeposit(g, tabs[0], 3e-11, btype, AbsorbArbitraryCutCell(g, P), bCellTable=tabs[1])
+        torch.cuda.synchronize()
+        got.append((P.getParticleData(), P.getIsInside(), *P.getChargeOnGridFixed()))
+    (pa, ina, fa, sa), (pb, inb, fb, sb) = got
+    assert sa == sb and np.array_equal(fa, fb) and 0 < ina.sum() < n
+    assert np.array_equal(pa[order], pb) and np.array_equal(ina[order], inb)
+    q = np.rint(rows[ina == 1, 5].astype(np.float32).astype(np.float64) * sa)
+    assert q.min() < 2.0 ** 40 < q.max() and int(fa.sum()) == sum(int(x) for x in q)
