@@ -331,7 +331,7 @@ int oec_secelec_emit(const oec_secelec_t *params, const double *rows_dev, const 
                      void *stream);
 
 /* Bytes of `work_dev` oec_furman_emit needs for `cap` absorbed rows
- * (cap <= 2^26; -1 beyond). */
+ * (cap <= 2^26; -1 beyond), at any multiple of 8 bytes. */
 int64_t oec_furman_work_bytes(int32_t cap);
 
 /* generateSecondaries (particleEmitter.pyx:154-308) on the absorbed rows at
@@ -374,7 +374,9 @@ int oec_step_advance(int32_t *step_dev, void *stream);
 
 /* --------------------------------------- particle management (A10, A25-A27) */
 
-/* Bytes of the work buffer of oec_sort_particles / oec_cell_merge. */
+/* Bytes of the work buffer of oec_sort_particles / oec_cell_merge: 48 per
+ * particle (32 of them rows through which particles in random order are moved)
+ * and 1 KB per 4096 particles. */
 int64_t oec_sort_work_bytes(int64_t capacity);
 
 /* sortByColumn (particles.pyx:49-50, :431-459): stable radix sort of the

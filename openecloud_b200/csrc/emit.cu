@@ -194,8 +194,8 @@ __device__ __forceinline__ void put_secondary(const double *r, double n0, double
 // (specfun.cuh), and with few rows the functions run side by side.  Which lane takes which
 // does not enter its value.  106,457 absorbed rows of 200 eV electrons (179,048
 // secondaries) on a B200: 3340 us for a thread per (row, slot) with the plain
-// inverses and a thread per row for the directions, 132 us this way; 250 secondaries
-// (one buildup step): 40 us, the latency of one inverse.
+// inverses and a thread per row for the directions, 95 us this way; 250 secondaries
+// (one buildup step): 25 us, the latency of one inverse.
 constexpr int kSplitT = 256, kSplitRows = 1024;
 constexpr int kKinds = 9;  // lone, gamma, and the kinds of sf::BetaConst
 

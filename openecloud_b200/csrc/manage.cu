@@ -5,9 +5,10 @@
 // Reference: particles.pyx sortByColumn (:49-50, :431-459),
 // particleManagement.pyx globalRandom (:35-67) and localRandom (:74-238).
 //  * Sorting is a stable least-significant-digit radix sort of 32-bit keys
-//    (8-bit digits): per pass a per-tile digit histogram, one exclusive scan
-//    over (digit, tile), and a stable scatter in which each tile ranks its
-//    elements by 1-bit split passes.
+//    (8-bit digits): per pass a per-tile digit histogram, one launch that scans
+//    each digit's tile counts (a CTA per digit), and a stable scatter in which
+//    a tile ranks its elements by warp votes and puts them in order in shared
+//    memory before they are written.
 //  * globalRandom removes n - target particles chosen uniformly without
 //    replacement (each thread throws darts at free slots with atomicOr on the
 //    removal bitmask, as the reference redraws until it hits a particle it has

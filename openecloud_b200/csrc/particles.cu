@@ -660,7 +660,7 @@ __global__ void k_push_begin(int32_t *n_absorbed, unsigned long long *__restrict
 // chunk lie within half a window of rows.  A sorted store passes, one in the
 // order of a run (loaded at random, refilled hole by hole) does not: with two
 // samples instead of four 3 % of the CTAs of a 512-row grid passed by chance
-// and held up the rest (2^24 electrons: 362 against 335 us).
+// and held up the rest (2^24 electrons: 8 % slower).
 __device__ __forceinline__ bool chunk_is_local(const FusedArgs &a, int n) {
     const int base = (int)blockIdx.x * kChunk;
     if (base >= n) return true;  // no chunk for this CTA: an empty store has no cell to read
@@ -682,8 +682,8 @@ __device__ __forceinline__ bool chunk_is_local(const FusedArgs &a, int n) {
 // outside, each lane's four adds to four cells of its own.  A CTA whose first
 // chunk is not local therefore goes without windows and barriers and adds in
 // lane pairs (add_pairs).  Per step against windows everywhere: 2^24 electrons in
-// random order on 512^2 427 -> 335 us, 2.2e6 on 1024^2 73 -> 57 us, 1e6 with a
-// gathered B on 300 x 240 58 -> 43 us; sorted 2^24 unchanged.  The two loops are
+// random order on 512^2 428 -> 322 us, 2.2e6 on 1024^2 73 -> 54 us, 1e6 with a
+// gathered B on 300 x 240 58 -> 38 us; sorted 2^24 unchanged.  The two loops are
 // kept apart: with the choice made per chunk inside one loop the sorted case lost
 // 2.5 %.
 template <int TB, int KIND, bool DEP>
