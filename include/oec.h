@@ -376,8 +376,14 @@ int oec_step_advance(int32_t *step_dev, void *stream);
 
 /* Bytes of the work buffer of oec_sort_particles / oec_cell_merge: 48 per
  * particle (32 of them rows through which particles in random order are moved)
- * and 1 KB per 4096 particles. */
+ * and 1 KB per 4096 particles.  Work and passes follow from the capacity that the
+ * call is given: a store with room for many more particles than it holds may be
+ * passed with a smaller capacity, any multiple of 1024 not below its count. */
 int64_t oec_sort_work_bytes(int64_t capacity);
+
+/* Bytes that suffice for oec_sort_particles by cell index (column 6), which
+ * needs no such rows. */
+int64_t oec_cell_sort_work_bytes(int64_t capacity);
 
 /* sortByColumn (particles.pyx:49-50, :431-459): stable radix sort of the
  * particles by column 2..5 (vx, vy, vz, w) or 6 (cell index); the sorted

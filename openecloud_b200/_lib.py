@@ -94,12 +94,12 @@ SIGNATURES = {
     "oec_step_advance": [_P, _P],
     "oec_bound_violations": [_P, _I32],
 }
-_INT64_RETURNING = {"oec_sort_work_bytes": [_I64]}
+_INT64_RETURNING = {"oec_sort_work_bytes": [_I64], "oec_cell_sort_work_bytes": [_I64]}
 
 _lib = None
 # entry points whose ctypes signatures live next to their Python users
 # (structure arguments defined there); registered at import of that module
-OTHER_DECLARED = {"oec_sort_work_bytes"}
+OTHER_DECLARED = {"oec_sort_work_bytes", "oec_cell_sort_work_bytes"}
 
 
 def lib():

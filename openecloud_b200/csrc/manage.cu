@@ -635,10 +635,14 @@ static bool vp2(const oec_particles_t *p) {
     return p && p->cell && p->ox && p->oy && p->vx && p->vy && p->vz && p->w && p->count && p->capacity > 0;
 }
 
-extern "C" int64_t oec_sort_work_bytes(int64_t capacity) {
+extern "C" int64_t oec_cell_sort_work_bytes(int64_t capacity) {
     int64_t tiles = (capacity + kTile - 1) / kTile;
-    // keys, vals (twice) | histogram | 256-byte slack (merge counters) | digit totals | rows of 32 bytes, aligned
-    return 4 * capacity * 4 + 256 * tiles * 4 + 256 + 4 * 256 + 32 * capacity + 256;
+    // keys, vals (twice) | histogram | 256-byte slack (merge counters) | digit totals
+    return 4 * capacity * 4 + 256 * tiles * 4 + 256 + 4 * 256;
+}
+
+extern "C" int64_t oec_sort_work_bytes(int64_t capacity) {
+    return oec_cell_sort_work_bytes(capacity) + 32 * capacity + 256;  // rows of 32 bytes, aligned
 }
 
 // The digit totals, behind the histogram and its 256-byte slack.

@@ -20,6 +20,7 @@ import torch
 from . import _lib
 from . import device as D
 from .constants import c
+from .particles import CHUNK
 
 WEIGHT_SUMS_CTAS = 1024  # OEC_WEIGHT_SUMS_CTAS: places per sum in the scratch of oec_weight_sums
 
@@ -84,7 +85,8 @@ def localRandom(gridObj, particlesObj, particleBoundaryObj, targetMacroParticleC
     goal = meanWeight * n / target
     maxT, minT = thresholdFactor * goal, goal / thresholdFactor
     ds = min(gridObj.getDx(), gridObj.getDy())
-    P.sortByColumn(5)
+    cap = D.round_up(max(n, 1), CHUNK)
+    P._sort(5, cap)
     # the two _searchSorted thresholds on the device: 8 bytes come back
     # instead of the weight array
     thr = D.zeros(2, torch.int32)
@@ -115,11 +117,12 @@ def localRandom(gridObj, particlesObj, particleBoundaryObj, targetMacroParticleC
     n_cand = min(n - to_split, max(0, int(oversample * to_merge)))
     n_cand -= n_cand % 2
     if to_merge > 0 and n_cand >= 2:
-        work = D.empty(int(_lib.lib().oec_sort_work_bytes(P._cap)), torch.uint8)
+        p = P.c_particles()
+        p.capacity = cap
         counters = D.zeros(2, torch.int32)
-        _lib.call("oec_cell_merge", gridObj.c_grid(), P.c_particles(), n_cand, to_merge, lam, factorDisLimit * ds,
+        _lib.call("oec_cell_merge", gridObj.c_grid(), p, n_cand, to_merge, lam, factorDisLimit * ds,
                   int(mergeScheme), int(seed), _next_call() if call is None else int(call), 3.0 * vt, P._mask.data_ptr(), counters.data_ptr(),
-                  work.data_ptr(), s)
+                  P._sort_area(cap).data_ptr(), s)
         localRandom.last_counters = counters.cpu().numpy()
     P.addAndRemoveParticles(rows[:to_split], None)
     localRandom.last_counts = (to_merge, to_split)

@@ -184,12 +184,25 @@ class Particles:
             col = 6  # x, y: the cell-major order is the position order used on the device
         if col not in (2, 3, 4, 5, 6):
             raise ValueError("column must be 0..5 (or 6 for cells)")
-        tmp = self.c_scratch()
-        if getattr(self, "_sort_work", None) is None or self._sort_work_cap != self._cap:
-            self._sort_work = D.empty(int(_lib.lib().oec_sort_work_bytes(self._cap)), torch.uint8)
-            self._sort_work_cap = self._cap
-        _lib.call("oec_sort_particles", self.c_particles(), tmp, col, self._sort_work.data_ptr(), D.stream())
+        self._sort(col, self._cap)
+
+    def _sort(self, col, cap):
+        """Sorts the store as one of capacity `cap`, at least its count: passes and work
+        area follow from that (a buildup's store has room for many times its particles)."""
+        p, tmp = self.c_particles(), self.c_scratch()
+        p.capacity = tmp.capacity = cap
+        _lib.call("oec_sort_particles", p, tmp, col, self._sort_area(cap, col).data_ptr(), D.stream())
         self._soa, self._sort_tmp = self._sort_tmp, self._soa
+
+    def _sort_area(self, cap, col=5):
+        """The work area of a sort by `col` or a merge at capacity `cap`, kept, and grown a
+        quarter ahead (up to what the whole store takes)."""
+        L = _lib.lib()
+        size = L.oec_cell_sort_work_bytes if col == 6 else L.oec_sort_work_bytes
+        if getattr(self, "_sort_work", None) is None or self._sort_work.shape[0] < size(cap):
+            self._sort_work = None
+            self._sort_work = D.empty(int(size(max(cap, min(self._cap, D.round_up(cap * 1.25, CHUNK))))), torch.uint8)
+        return self._sort_work
 
     def c_scratch(self):
         """A second store of the same capacity: the sort's output (swapped in

@@ -281,3 +281,35 @@ def test_weight_sums(gpu, n):
     want = math.fsum(w), math.fsum((v[0] ** 2 + v[1] ** 2 + v[2] ** 2) * w * w)
     assert all(np.array_equal(x, got[0]) for x in got)
     assert np.allclose(got[0], want, rtol=2e-14, atol=0)
+
+
+def test_merge_memory_follows_the_particles(gpu):
+    """A merge in a store with room for 200 times its particles takes memory for the
+    particles (48 bytes each and a quarter ahead for the work area, 48 each for split rows, and less
+    than 4 MB beside that), not for the room, and leaves the rows of a store that is full."""
+    import torch
+    from openecloud_b200.grid import Grid
+    from openecloud_b200.particleBoundary import AbsorbElliptical
+    from openecloud_b200.particleManagement import localRandom
+    from openecloud_b200.particles import Particles
+    rng = np.random.default_rng(4)
+    n, rows = 20_000, []
+    pd = np.empty((n, 6))
+    pd[:, 0:2] = rng.uniform(-0.012, 0.012, (n, 2))
+    pd[:, 2:5] = rng.normal(0, 1e6, (n, 3))
+    pd[:, 5] = rng.uniform(0.5, 2.0, n)
+    g = Grid(64, 64, 0.04, 0.04, 1)
+    for cap in (4_000_000, n):
+        P = Particles("electrons", "variableWeight", capacity=cap)
+        P.setParticleData(pd)
+        P._bind(g)
+        P.c_scratch()  # the store's own second half and index, for its room as before
+        P._hole_buffers()
+        bd = AbsorbElliptical(g, P)
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        localRandom(g, P, bd, n - n // 10, seed=3, call=1)
+        assert torch.cuda.max_memory_allocated() - before < (48 * 1.25 + 48) * n + (4 << 20)
+        rows.append(P.getParticleData())
+    assert len(rows[0]) < n and np.array_equal(rows[0], rows[1])

@@ -29,3 +29,26 @@ def test_sort_is_stable_at_tile_edges(gpu, n, col):
     P.sortByColumn(col)
     for k, v in P.soa().items():
         assert np.array_equal(v[:n].cpu().numpy().view(np.uint32), soa[k][order].view(np.uint32)), k
+
+
+@pytest.mark.parametrize("n", [1, 4097, 12_289])
+def test_cell_sort_stays_in_its_work_area(gpu, n):
+    """oec_cell_sort_work_bytes suffices for a sort by cell: what lies behind is untouched."""
+    import torch
+    from openecloud_b200 import _lib
+    from openecloud_b200 import device as D
+    from openecloud_b200.grid import Grid
+    from openecloud_b200.particles import Particles
+    rng = np.random.default_rng(n)
+    P = Particles("electrons", "variableWeight")
+    pd = np.ones((n, 6))
+    pd[:, 0:2] = rng.uniform(-0.0199, 0.0199, (n, 2))
+    P.setParticleData(pd)
+    P._bind(Grid(70, 90, 0.04, 0.04, 0))
+    cell = P.soa()["cell"][:n].cpu().numpy()
+    size = int(_lib.lib().oec_cell_sort_work_bytes(P._cap))
+    area = torch.full((size + 4096,), 0x5a, dtype=torch.uint8, device="cuda")
+    tmp = P.c_scratch()
+    _lib.call("oec_sort_particles", P.c_particles(), tmp, 6, area.data_ptr(), D.stream())
+    assert bool((area[size:] == 0x5a).all())
+    assert np.array_equal(P._sort_tmp["cell"][:n].cpu().numpy(), np.sort(cell))
